@@ -211,10 +211,6 @@ int zc_moe_create(const zc_moe_desc* desc, int device, zc_moe** out) {
     A(&c.logits, T * E * 4); A(&c.gate_logit, T * 4); A(&c.ids, T * K * 4); A(&c.weights, T * K * 4);
     A(&c.offsets, (E + 1) * 4); A(&c.perm, T * K * 4); A(&c.active, E * 4); A(&c.items, E * 16); A(&c.counters, (16 + size_t(d.layers)) * 4);
     if (T * K > 4096) A(&m->permute_blocks, permute_block_count(T * K) * E * 4);
-    A(&m->router_partial, 16 * T * size_t(router_rows_padded(d)) * 4);
-    const size_t done_n = size_t(router_rows_padded(d) / 32) * ((T + 7) / 8);
-    A(&m->router_done, done_n * 4);
-    if (rc == ZC_OK && (e = cudaMemset(m->router_done, 0, done_n * 4)) != cudaSuccess) rc = cuda_fail(m, e, "cudaMemset");
     A(&c.hbuf, (T * K + T) * F * 4);
     if (prefill_supported(d) && T > 64) {
         A(&m->xp, T * H * 2); A(&m->hbuf16, (T * K + T) * F * 2);
@@ -910,10 +906,7 @@ int zc_moe_set_option(zc_moe* m, const char* name, int value) {
     }
     if (!std::strcmp(name, "router_db")) {
         if (value != 0 && value != 1) return fail(m, ZC_EINVAL, "router_db must be 0 or 1");
-        DeviceGuard guard(m->device);
-        drop_graphs(m);
-        m->router_db = uint32_t(value);
-        return ZC_OK;
+        return ZC_OK;                        // both forms it chose between are one kernel now
     }
     if (!std::strcmp(name, "meta_blocks")) {
         if (value < 0 || value > 3) return fail(m, ZC_EINVAL, "meta_blocks must be 0..3");

@@ -233,7 +233,6 @@ struct zc_moe {
     int32_t* pf_ntiles = nullptr;
     int32_t* permute_blocks = nullptr;   // [ceil(max slots / 2048)][E]: per-CTA expert counts of the multi-CTA permutation
     uint32_t pf_max_tiles = 0;
-    uint32_t* router_done = nullptr;     // arrival counters of the router's (row tile, token tile) pairs
     zc::Call ep{};                       // second scratch set: the experts step of expert parallelism (rows from all ranks)
     uint32_t ep_rows_cap = 0;
     // peer transport of expert parallelism (allocated when local_experts < experts; usable after zc_moe_ep_attach)
@@ -249,7 +248,6 @@ struct zc_moe {
     const int32_t* cancel = nullptr;      // host flag read before a layer is issued (zc_moe_set_cancel)
     int4* empty_items = nullptr;         // an item list with no entries (launches that run the shared expert only)
     int32_t* zero_counters = nullptr;    // an always-zero counter block (launches that run the shared expert only)
-    float* router_partial = nullptr;     // [16, max_tokens, rows_padded] partition sums of the router
     void* act[2] = {nullptr, nullptr};   // stack ping-pong activations [max_tokens, H]
     void* host_x = nullptr;       // pinned staging for the host entry points
     void* host_out = nullptr;
@@ -269,7 +267,6 @@ struct zc_moe {
     uint32_t pdl = 0xffffffffu;   // bit per KernelKind: that kernel launches with programmatic stream serialization (see launch_chained)
     bool exact_h = false;         // down reads the FP32 SwiGLU rows as two FP16 terms instead of one
     uint32_t few_tiles_gate_up = 1, few_tiles_down = 2;      // 16-row tiles per warp of the streaming launches for those experts (few items: more, shorter CTAs)
-    uint32_t router_db = 1;              // long batches: double-buffered whole-K router tiles (FP32 router rows, BF16 activations)
     uint32_t meta_blocks = 1;            // streaming kernels fetch scales and biases eight groups at a time: 0 never, 1 for gate/up with long rows, 2 wherever possible
     uint32_t prefill_small_rows = 16;   // long batches: experts with at most this many rows run on the streaming kernels (0 = none)
     bool prefill_wide = true;     // long batches: wide-tile kernel with accumulators resident in TMEM (false: per-group drain kernel)
@@ -283,7 +280,6 @@ namespace zc {
 // Launchers (each returns the number of kernels launched, or a negative ZC_* code with moe->error set).
 int launch_router(zc_moe* m, const Call& c, cudaStream_t s);
 int launch_router_partial(zc_moe* m, const Call& c, cudaStream_t s);
-uint32_t router_rows_padded(const zc_moe_desc& d);
 int launch_route_permute(zc_moe* m, const Call& c, cudaStream_t s, bool do_route, bool do_permute);
 int launch_forced_weights(zc_moe* m, const Call& c, const int32_t* forced, cudaStream_t s);
 int launch_experts_decode(zc_moe* m, const Call& c, cudaStream_t s);

@@ -8,9 +8,9 @@
 // because one last-bit change in a logit can flip a top-k decision; it reproduces the MLX bit patterns
 // the reference's own test holds (tests/test_qwen.cpp:798-826).
 //
-// router_partial_kernel: grid (row tiles of 32, 16 partitions, token tiles). A CTA stages its slice of
-// x (k-major) and of the router rows (k-major) in shared memory, then every thread runs its chains:
-// TT = 64: 4 tokens x 2 rows per thread; TT = 8: one (token, row) per thread.
+// router_partial_kernel (the entry point that may not allocate): grid (row tiles of 32, 16 partitions, token tiles). A CTA
+// stages its slice of x (k-major) and of the router rows (k-major) in shared memory, then every thread runs its chains.
+// Layer calls use router_cluster_kernel up to 128 tokens and router_tile_kernel beyond.
 #include "common.cuh"
 #include <cooperative_groups.h>
 
@@ -18,14 +18,12 @@ namespace zc {
 namespace {
 
 constexpr int ROUTER_THREADS = 256;
-constexpr int ROW_TILE_PAD = 64;      // rows are padded to a multiple of this in the partials buffer
 
-// TT tokens x ROW_TILE rows per CTA: TT = 8 -> 32 rows (one output per thread), TT = 16 -> 32 rows (two),
-// TT = 32 -> 64 rows (four tokens x two rows per thread: eight chains share two shared-memory reads per k).
+// TT tokens x 32 rows per CTA: TT = 8 -> one output per thread, TT = 16 -> two.
 template <int TT>
 __global__ void __launch_bounds__(ROUTER_THREADS) router_partial_kernel(Call c, float* __restrict__ partial, uint32_t rows_padded,
                                                                          uint32_t* __restrict__ tile_done, uint32_t reduce) {
-    constexpr int ROW_TILE = TT == 32 ? 64 : 32;
+    constexpr int ROW_TILE = 32;
     extern __shared__ __align__(16) float smem[];
     const uint32_t H = c.H, part = H / 16;
     float* xs = smem;                    // [part][TT]
@@ -96,45 +94,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) router_partial_kernel(Call c, 
     }
     __syncthreads();
 
-    if constexpr (TT == 64) {
-        const uint32_t tx = tid % 16, ty = tid / 16;        // rows 2tx, 2tx+1; tokens 4ty .. 4ty+3
-        float acc[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0f;
-#pragma unroll 4
-        for (uint32_t k = 0; k < part; ++k) {
-            const float4 xv = *reinterpret_cast<const float4*>(xs + k * TT + ty * 4);
-            const float2 wv = *reinterpret_cast<const float2*>(ws + k * ROW_TILE + tx * 2);
-            acc[0][0] = __fmaf_rn(xv.x, wv.x, acc[0][0]); acc[0][1] = __fmaf_rn(xv.x, wv.y, acc[0][1]);
-            acc[1][0] = __fmaf_rn(xv.y, wv.x, acc[1][0]); acc[1][1] = __fmaf_rn(xv.y, wv.y, acc[1][1]);
-            acc[2][0] = __fmaf_rn(xv.z, wv.x, acc[2][0]); acc[2][1] = __fmaf_rn(xv.z, wv.y, acc[2][1]);
-            acc[3][0] = __fmaf_rn(xv.w, wv.x, acc[3][0]); acc[3][1] = __fmaf_rn(xv.w, wv.y, acc[3][1]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t t = t0 + ty * 4 + i;
-            if (t < c.T) *reinterpret_cast<float2*>(partial + (size_t(p) * c.T + t) * rows_padded + e0 + tx * 2) = make_float2(acc[i][0], acc[i][1]);
-        }
-    } else if constexpr (TT == 32) {
-        const uint32_t tx = tid % 32, ty = tid / 32;        // rows 2tx, 2tx+1; tokens 4ty .. 4ty+3
-        float acc[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0f;
-#pragma unroll 4
-        for (uint32_t k = 0; k < part; ++k) {
-            const float4 xv = *reinterpret_cast<const float4*>(xs + k * TT + ty * 4);
-            const float2 wv = *reinterpret_cast<const float2*>(ws + k * ROW_TILE + tx * 2);
-            acc[0][0] = __fmaf_rn(xv.x, wv.x, acc[0][0]); acc[0][1] = __fmaf_rn(xv.x, wv.y, acc[0][1]);
-            acc[1][0] = __fmaf_rn(xv.y, wv.x, acc[1][0]); acc[1][1] = __fmaf_rn(xv.y, wv.y, acc[1][1]);
-            acc[2][0] = __fmaf_rn(xv.z, wv.x, acc[2][0]); acc[2][1] = __fmaf_rn(xv.z, wv.y, acc[2][1]);
-            acc[3][0] = __fmaf_rn(xv.w, wv.x, acc[3][0]); acc[3][1] = __fmaf_rn(xv.w, wv.y, acc[3][1]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t t = t0 + ty * 4 + i;
-            if (t < c.T) *reinterpret_cast<float2*>(partial + (size_t(p) * c.T + t) * rows_padded + e0 + tx * 2) = make_float2(acc[i][0], acc[i][1]);
-        }
-    } else if constexpr (TT == 16) {
+    if constexpr (TT == 16) {
         const uint32_t tx = tid % 16, ty = tid / 16;        // rows 2tx, 2tx+1; token ty
         float a0 = 0.0f, a1 = 0.0f;
 #pragma unroll 8
@@ -417,366 +377,271 @@ int launch_router_cluster(zc_moe* m, const Call& c, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Long batches: one CTA owns a 64-token x 64-row tile of the logits for the whole of K. It walks the sixteen
-// partitions in order; inside a partition every (token, row) pair is the k-ascending chain of fused multiply-adds,
-// and the finished partial is added to the pair's running total - the same additions in the same order as the
-// partition kernels above ("partials added 0..15 starting from zero"), but nothing leaves the registers: no partial
-// store, no arrival counter, no ordered re-read. Thread (tx, ty) holds rows tx + 16 i and tokens 4 ty + j (i, j < 4):
-// sixteen independent chains, fed by four row reads and four broadcast token reads per four k, which keeps the
-// kernel bound by the FP32 pipe and not by shared memory. Tiles keep the row-major [row][k] layout (leading
-// dimension part + 4 floats), so FP32 router rows are copied with 16-byte cp.async.
-constexpr int LONG_TT = 64, LONG_RT = 64;
-#ifndef ZC_RL_ROWS
-#define ZC_RL_ROWS 4          // rows x tokens per thread: 4 x 4 chains, 256 threads (8 x 4 with 128 threads measured 20 % slower)
-#endif
-#ifndef ZC_RL_UNROLL
-#define ZC_RL_UNROLL 2
-#endif
-#ifndef ZC_RL_BLOCKS
-#define ZC_RL_BLOCKS 2
-#endif
-#define ZC_PRAGMA(x) _Pragma(#x)
-#define ZC_UNROLL(n) ZC_PRAGMA(unroll n)
-constexpr int LONG_RI = ZC_RL_ROWS, LONG_TJ = 4;
-constexpr int LONG_TXN = LONG_RT / LONG_RI, LONG_TYN = LONG_TT / LONG_TJ, LONG_THREADS = LONG_TXN * LONG_TYN;
-// Thread (tx, ty) owns rows tx + TXN i and tokens ty + TYN j: the lanes of a warp read consecutive rows of either tile,
-// which the row pitch of part + 4 floats spreads over all banks (one wavefront per 128 distinct bytes).
-__global__ void __launch_bounds__(LONG_THREADS, ZC_RL_BLOCKS) router_long_kernel(Call c) {
-    extern __shared__ __align__(16) float smem[];
-    const uint32_t H = c.H, part = H / 16, LD = part + 4;
-    float* ws = smem;                       // [LONG_RT][LD]
-    float* xs = ws + LONG_RT * LD;          // [LONG_TT][LD]
-    const uint32_t e0 = blockIdx.x * LONG_RT, t0 = blockIdx.y * LONG_TT;
-    const uint32_t rows_total = c.E + (c.has_shared ? 1u : 0u);
-    const uint32_t tid = threadIdx.x, tx = tid % LONG_TXN, ty = tid / LONG_TXN, warp = tid / 32, lane = tid % 32;
-    const bool x32 = c.act_dtype == ZC_F32, w32 = c.router_dtype == ZC_F32;
-    const uint32_t rows_here = min(uint32_t(LONG_RT), rows_total - e0);
-    const bool narrow = rows_here <= LONG_THREADS / LONG_TT;
-    float total[LONG_RI][LONG_TJ];
-#pragma unroll
-    for (int i = 0; i < LONG_RI; ++i)
-#pragma unroll
-        for (int j = 0; j < LONG_TJ; ++j) total[i][j] = 0.0f;
-    pdl_wait();
-    for (uint32_t p = 0; p < 16; ++p) {
-        const uint32_t k0 = p * part;
-        __syncthreads();                     // the previous partition's tiles have been consumed
-        // Staging without divisions: warp w copies rows w, w + warps, ... of both tiles, its lanes walk the row.
-        for (uint32_t el = warp; el < (narrow ? rows_here : uint32_t(LONG_RT)); el += LONG_THREADS / 32) {
-            const uint32_t e = e0 + el;
-            float* dst = ws + el * LD;
-            if (e >= rows_total) {
-                for (uint32_t kq = lane; kq < part / 4; kq += 32) *reinterpret_cast<float4*>(dst + kq * 4) = make_float4(0, 0, 0, 0);
-            } else if (w32) {
-                const float* base = (e < c.E ? static_cast<const float*>(c.router_w) + size_t(e) * H : static_cast<const float*>(c.shared_gate_w)) + k0;
-                for (uint32_t kq = lane; kq < part / 4; kq += 32) cp_async16(dst + kq * 4, base + kq * 4);
-            } else {
-                const uint16_t* base = (e < c.E ? static_cast<const uint16_t*>(c.router_w) + size_t(e) * H : static_cast<const uint16_t*>(c.shared_gate_w)) + k0;
-                for (uint32_t kq = lane; kq < part / 4; kq += 32) {
-                    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(base + kq * 4));
-                    *reinterpret_cast<float4*>(dst + kq * 4) = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
-                                                                           __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
-                }
-            }
-        }
-        if (x32) {
-            for (uint32_t tt = warp; tt < LONG_TT; tt += LONG_THREADS / 32) {
-                const uint32_t t = t0 + tt;
-                float* dst = xs + tt * LD;
-                if (t < c.T) { const float* base = static_cast<const float*>(c.x) + size_t(t) * H + k0; for (uint32_t kq = lane; kq < part / 4; kq += 32) cp_async16(dst + kq * 4, base + kq * 4); }
-                else for (uint32_t kq = lane; kq < part / 4; kq += 32) *reinterpret_cast<float4*>(dst + kq * 4) = make_float4(0, 0, 0, 0);
-            }
-        } else {
-            // BF16 rows: 16 bytes = eight values per lane; a half-warp takes a row (two rows per pass of the warp)
-            for (uint32_t tt = warp * 2 + lane / 16; tt < LONG_TT; tt += LONG_THREADS / 16) {
-                const uint32_t t = t0 + tt;
-                const uint16_t* base = static_cast<const uint16_t*>(c.x) + size_t(t) * H + k0;
-                for (uint32_t kb = lane % 16; kb < part / 8; kb += 16) {
-                    uint4 raw = make_uint4(0, 0, 0, 0);
-                    if (t < c.T) raw = __ldcg(reinterpret_cast<const uint4*>(base + kb * 8));
-                    float4* dst = reinterpret_cast<float4*>(xs + tt * LD + kb * 8);
-                    dst[0] = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
-                    dst[1] = make_float4(__uint_as_float(raw.z << 16), __uint_as_float(raw.z & 0xffff0000u), __uint_as_float(raw.w << 16), __uint_as_float(raw.w & 0xffff0000u));
-                }
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        if (narrow) {
-            // A row tile with one or two rows (the shared gate's row after 512 experts): one chain per thread,
-            // thread = (token, row), the same k-ascending chain and the same ordered sum of partials.
-            const uint32_t tt = tid % LONG_TT, rr = tid / LONG_TT;
-            float a = 0.0f;
-            if (rr < rows_here) {
-                const float* wr = ws + rr * LD;
-                const float* xr = xs + tt * LD;
-                for (uint32_t k = 0; k < part; k += 4) {
-                    const float4 wv = *reinterpret_cast<const float4*>(wr + k), xv = *reinterpret_cast<const float4*>(xr + k);
-                    a = __fmaf_rn(xv.x, wv.x, a);
-                    a = __fmaf_rn(xv.y, wv.y, a);
-                    a = __fmaf_rn(xv.z, wv.z, a);
-                    a = __fmaf_rn(xv.w, wv.w, a);
-                }
-            }
-            total[0][0] = __fadd_rn(total[0][0], a);
-            continue;
-        }
-        float acc[LONG_RI][LONG_TJ];
-#pragma unroll
-        for (int i = 0; i < LONG_RI; ++i)
-#pragma unroll
-            for (int j = 0; j < LONG_TJ; ++j) acc[i][j] = 0.0f;
-        const float* wrow = ws + tx * LD;
-        const float* xrow = xs + ty * LD;
-ZC_UNROLL(ZC_RL_UNROLL)
-        for (uint32_t k = 0; k < part; k += 4) {
-            float4 wv[LONG_RI], xv[LONG_TJ];
-#pragma unroll
-            for (int i = 0; i < LONG_RI; ++i) wv[i] = *reinterpret_cast<const float4*>(wrow + i * LONG_TXN * LD + k);
-#pragma unroll
-            for (int j = 0; j < LONG_TJ; ++j) xv[j] = *reinterpret_cast<const float4*>(xrow + j * LONG_TYN * LD + k);
-#pragma unroll
-            for (int i = 0; i < LONG_RI; ++i)
-#pragma unroll
-                for (int j = 0; j < LONG_TJ; ++j) {
-                    float a = acc[i][j];
-                    a = __fmaf_rn(xv[j].x, wv[i].x, a);
-                    a = __fmaf_rn(xv[j].y, wv[i].y, a);
-                    a = __fmaf_rn(xv[j].z, wv[i].z, a);
-                    a = __fmaf_rn(xv[j].w, wv[i].w, a);
-                    acc[i][j] = a;
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < LONG_RI; ++i)
-#pragma unroll
-            for (int j = 0; j < LONG_TJ; ++j) total[i][j] = __fadd_rn(total[i][j], acc[i][j]);      // partial p joins the ordered sum
-    }
-    pdl_launch_dependents();
-    if (narrow) {
-        const uint32_t tt = tid % LONG_TT, rr = tid / LONG_TT, e = e0 + rr, t = t0 + tt;
-        if (rr < rows_here && t < c.T) {
-            if (e < c.E) c.logits[size_t(t) * c.E + e] = c.router_bias ? __fadd_rn(total[0][0], c.router_bias[e]) : total[0][0];
-            else c.gate_logit[t] = total[0][0];
-        }
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < LONG_RI; ++i) {
-        const uint32_t e = e0 + tx + LONG_TXN * i;
-        if (e >= rows_total) continue;
-#pragma unroll
-        for (int j = 0; j < LONG_TJ; ++j) {
-            const uint32_t t = t0 + ty + LONG_TYN * j;
-            if (t >= c.T) continue;
-            if (e < c.E) c.logits[size_t(t) * c.E + e] = c.router_bias ? __fadd_rn(total[i][j], c.router_bias[e]) : total[i][j];
-            else c.gate_logit[t] = total[i][j];
-        }
-    }
+// Register-tiled form for more than 128 tokens. A CTA of 128 threads owns 64 tokens (128 in the widest form) x 64 rows of
+// the logits and `16 / ranks` consecutive partitions of K. The bound is the FP32 pipe: every logit is a pinned chain of
+// fused multiply-adds, 2 T E H flops whatever the schedule. Each thread runs 8 rows x TJ tokens of chains, two rows per
+// instruction: fma.rn.f32x2 is two independent IEEE fused multiply-adds on the halves of a 64-bit register, so every chain
+// keeps its own k-ascending order and its bits at half the issue slots, which the shared-memory reads and the duplicated
+// token operands need. Rows are stored in pairs ([row pair][k][2]: a 16-byte read is the operand of two k), tokens as FP32
+// [token][k], both padded so that the lanes of a warp (8 row groups x 4 token groups) read distinct banks. A chain's next
+// link comes 4 TJ instructions later (with 4 in between the FMA latency showed: 156 against 146 us at 2048 tokens). K
+// arrives in double-buffered chunks of 32: the next chunk is in registers while this one is multiplied.
+// ranks = 1: each finished partition is added to the tile's running total in shared memory - the additions "partials 0..15
+// in order, starting from zero" of the reference. ranks = 8 (too few tiles for the SMs): the CTAs of a cluster share the
+// partitions of a tile, keep every partial in shared memory, and after a cluster barrier each adds the sixteen partials of
+// its part of the tile in order, reading its peers' (DSMEM).
+// Measured against the forms it replaced (partials in global memory; 4 x 4 scalar chains): 513 tokens 77 -> 56 us, 256 tokens
+// at hidden 4096 85 -> 58, 2048 tokens 167 -> 146, 8192 tokens 604 -> 474 (51 % of the FP32 rate; a register tile of 8 x 4
+// needs 12 shared-memory wavefronts per 16 FMA instructions and would be bound by them at 66 %, 8 x 8 at 100 %; what is left
+// is the duplication of the token operand and the latency of the reads at two to three CTAs per SM).
+constexpr int RT_ROWS = 64, RT_THREADS = 128, RT_CHUNK = 32;
+constexpr int RT_WLD = RT_CHUNK * 2 + 4, RT_PLD = RT_ROWS + 8;      // pitches in floats: row pair, token of a partial tile
+// Geometry of a CTA with TJ tokens per thread.
+template <int TJ> struct RouterTile {
+    static constexpr int TOKENS = 16 * TJ;
+    static constexpr int XLD = RT_CHUNK + 4;                         // pitch of a token in floats
+    static constexpr int STAGE_FLOATS = (RT_ROWS / 2) * RT_WLD + TOKENS * XLD, PART_FLOATS = TOKENS * RT_PLD;
+};
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float4 bf16x4(uint2 raw) {
+    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
 }
 
-// The same whole-K tile for the common format - FP32 router rows, BF16 activations - with the two tiles double-buffered:
-// the activations stay BF16 in shared memory (they become FP32 in registers, the same values), so both tiles are plain
-// 16-byte cp.async copies, and partition p + 1 is fetched while partition p is multiplied. With one buffer the two CTAs
-// of an SM start together and stay in step, so the FMA pipe idles through every staging phase (ncu: FMA pipe 41 %).
-__global__ void __launch_bounds__(LONG_THREADS, 2) router_long_db_kernel(Call c) {
+template <bool X32, bool W32, int TJ>
+__global__ void __launch_bounds__(RT_THREADS, TJ == 8 ? 3 : 4) router_tile_kernel(Call c, uint32_t ranks) {
+    using Tile = RouterTile<TJ>;
+    constexpr int RT_TOKENS = Tile::TOKENS, RT_STAGE_FLOATS = Tile::STAGE_FLOATS, RT_PART_FLOATS = Tile::PART_FLOATS, XLD = Tile::XLD;
     extern __shared__ __align__(16) float smem[];
-    const uint32_t H = c.H, part = H / 16, LD = part + 4, LDH = part + 8;
-    const uint32_t w_floats = LONG_RT * LD, stage_bytes = w_floats * 4 + LONG_TT * LDH * 2;       // one stage: [64][LD] floats, then [64][LDH] halves
-    const uint32_t e0 = blockIdx.x * LONG_RT, t0 = blockIdx.y * LONG_TT;
-    const uint32_t rows_total = c.E + (c.has_shared ? 1u : 0u);
-    const uint32_t tid = threadIdx.x, tx = tid % LONG_TXN, ty = tid / LONG_TXN, warp = tid / 32, lane = tid % 32;
-    const uint32_t rows_here = min(uint32_t(LONG_RT), rows_total - e0);
-    const bool narrow = rows_here <= LONG_THREADS / LONG_TT;
-    auto ws_of = [&](uint32_t stage) { return reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(smem) + stage * stage_bytes); };
-    auto xh_of = [&](uint32_t stage) { return reinterpret_cast<uint16_t*>(reinterpret_cast<uint8_t*>(smem) + stage * stage_bytes + w_floats * 4); };
-    auto issue = [&](uint32_t p) {
-        const uint32_t k0 = p * part;
-        float* ws = ws_of(p & 1);
-        uint16_t* xh = xh_of(p & 1);
-        for (uint32_t el = warp; el < (narrow ? rows_here : uint32_t(LONG_RT)); el += LONG_THREADS / 32) {
-            const uint32_t e = e0 + el;
-            float* dst = ws + el * LD;
-            if (e >= rows_total) {
-                for (uint32_t kq = lane; kq < part / 4; kq += 32) *reinterpret_cast<float4*>(dst + kq * 4) = make_float4(0, 0, 0, 0);
-            } else {
-                const float* base = (e < c.E ? static_cast<const float*>(c.router_w) + size_t(e) * H : static_cast<const float*>(c.shared_gate_w)) + k0;
-                for (uint32_t kq = lane; kq < part / 4; kq += 32) cp_async16(dst + kq * 4, base + kq * 4);
+    const uint32_t H = c.H, part = H / 16, parts = 16 / ranks;
+    float* ps = smem + 2 * RT_STAGE_FLOATS;          // [parts][RT_TOKENS][RT_PLD] partials (ranks > 1), else one running total
+    const uint32_t cr = blockIdx.x, e0 = blockIdx.y * RT_ROWS, t0 = blockIdx.z * RT_TOKENS;
+    const uint32_t rows_total = c.E + (c.has_shared ? 1u : 0u), rows_here = min(uint32_t(RT_ROWS), rows_total - e0);
+    const uint32_t tid = threadIdx.x, rg = tid % 8, tg = tid / 8;
+    constexpr int NARROW_ROWS = RT_THREADS / RT_TOKENS;
+    const bool narrow = rows_here <= uint32_t(NARROW_ROWS);        // the shared gate's row on its own: one chain per thread
+    const uint32_t k_first = cr * parts * part, k_last = k_first + parts * part;
+
+    // Staging: a task is four k of a row pair, or eight k of a token. Two and two of them per thread and chunk.
+    constexpr int WT = (RT_ROWS / 2) * (RT_CHUNK / 4) / RT_THREADS, XT = RT_TOKENS * (RT_CHUNK / 8) / RT_THREADS;
+    float4 w[WT][2];
+    uint4 x[XT][X32 ? 2 : 1];
+    auto load_w = [&](uint32_t k, uint32_t n) {      // n: k of this chunk (a multiple of 8, at most RT_CHUNK)
+#pragma unroll
+        for (int u = 0; u < WT; ++u) {
+            const uint32_t kq = tid % (RT_CHUNK / 4), pr = tid / (RT_CHUNK / 4) + u * (RT_THREADS / (RT_CHUNK / 4));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t e = e0 + pr * 2 + h;
+                w[u][h] = make_float4(0, 0, 0, 0);
+                if (e >= rows_total || kq * 4 >= n) continue;
+                const void* base = e < c.E ? c.router_w : c.shared_gate_w;
+                const size_t at = size_t(e < c.E ? e : 0) * H + k + kq * 4;
+                if (W32) w[u][h] = __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + at));
+                else w[u][h] = bf16x4(__ldg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + at)));
             }
         }
-        for (uint32_t tt = warp * 2 + lane / 16; tt < LONG_TT; tt += LONG_THREADS / 16) {      // a half-warp takes a row of 16-byte pieces
-            const uint32_t t = t0 + tt;
-            const uint16_t* base = static_cast<const uint16_t*>(c.x) + size_t(t) * H + k0;
-            for (uint32_t kb = lane % 16; kb < part / 8; kb += 16) {
-                if (t < c.T) cp_async16(xh + tt * LDH + kb * 8, base + kb * 8);
-                else *reinterpret_cast<uint4*>(xh + tt * LDH + kb * 8) = make_uint4(0, 0, 0, 0);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto x4 = [](uint2 raw) { return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)); };
-    float total[LONG_RI][LONG_TJ];
+    auto load_x = [&](uint32_t k, uint32_t n) {
 #pragma unroll
-    for (int i = 0; i < LONG_RI; ++i)
+        for (int u = 0; u < XT; ++u) {
+            const uint32_t kb = tid % (RT_CHUNK / 8), t = t0 + tid / (RT_CHUNK / 8) + u * (RT_THREADS / (RT_CHUNK / 8));
+            const bool on = t < c.T && kb * 8 < n;
+            const uint4* p = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(c.x) + (size_t(t) * H + k + kb * 8) * (X32 ? 4 : 2));
 #pragma unroll
-        for (int j = 0; j < LONG_TJ; ++j) total[i][j] = 0.0f;
-    pdl_wait();
-    issue(0);
-    for (uint32_t p = 0; p < 16; ++p) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                     // partition p has landed for everyone, and partition p - 1 has been consumed
-        if (p + 1 < 16) issue(p + 1);        // into the buffer partition p - 1 used
-        const float* ws = ws_of(p & 1);
-        const uint16_t* xh = xh_of(p & 1);
-        if (narrow) {
-            const uint32_t tt = tid % LONG_TT, rr = tid / LONG_TT;
-            float a = 0.0f;
-            if (rr < rows_here) {
-                const float* wr = ws + rr * LD;
-                for (uint32_t k = 0; k < part; k += 4) {
-                    const float4 wv = *reinterpret_cast<const float4*>(wr + k), xv = x4(*reinterpret_cast<const uint2*>(xh + tt * LDH + k));
-                    a = __fmaf_rn(xv.x, wv.x, a);
-                    a = __fmaf_rn(xv.y, wv.y, a);
-                    a = __fmaf_rn(xv.z, wv.z, a);
-                    a = __fmaf_rn(xv.w, wv.w, a);
-                }
+            for (int h = 0; h < (X32 ? 2 : 1); ++h) x[u][h] = on ? __ldcg(p + h) : make_uint4(0, 0, 0, 0);
+        }
+    };
+    auto store = [&](float* stage) {
+        float* ws = stage;
+        float* xs = stage + (RT_ROWS / 2) * RT_WLD;
+#pragma unroll
+        for (int u = 0; u < WT; ++u) {
+            const uint32_t kq = tid % (RT_CHUNK / 4), pr = tid / (RT_CHUNK / 4) + u * (RT_THREADS / (RT_CHUNK / 4));
+            float4* to = reinterpret_cast<float4*>(ws + pr * RT_WLD + kq * 8);
+            to[0] = make_float4(w[u][0].x, w[u][1].x, w[u][0].y, w[u][1].y);
+            to[1] = make_float4(w[u][0].z, w[u][1].z, w[u][0].w, w[u][1].w);
+        }
+#pragma unroll
+        for (int u = 0; u < XT; ++u) {
+            const uint32_t kb = tid % (RT_CHUNK / 8), tt = tid / (RT_CHUNK / 8) + u * (RT_THREADS / (RT_CHUNK / 8));
+            if constexpr (X32) {
+                uint4* to = reinterpret_cast<uint4*>(xs + tt * XLD + kb * 8);
+                to[0] = x[u][0]; to[1] = x[u][X32 ? 1 : 0];
+            } else {
+                float4* to = reinterpret_cast<float4*>(xs + tt * XLD + kb * 8);
+                to[0] = bf16x4(make_uint2(x[u][0].x, x[u][0].y)); to[1] = bf16x4(make_uint2(x[u][0].z, x[u][0].w));
             }
-            total[0][0] = __fadd_rn(total[0][0], a);
-            continue;
         }
-        float acc[LONG_RI][LONG_TJ];
-#pragma unroll
-        for (int i = 0; i < LONG_RI; ++i)
-#pragma unroll
-            for (int j = 0; j < LONG_TJ; ++j) acc[i][j] = 0.0f;
-        const float* wrow = ws + tx * LD;
-#pragma unroll 2
-        for (uint32_t k = 0; k < part; k += 4) {
-            float4 wv[LONG_RI], xv[LONG_TJ];
-#pragma unroll
-            for (int i = 0; i < LONG_RI; ++i) wv[i] = *reinterpret_cast<const float4*>(wrow + i * LONG_TXN * LD + k);
-#pragma unroll
-            for (int j = 0; j < LONG_TJ; ++j) xv[j] = x4(*reinterpret_cast<const uint2*>(xh + (ty + j * LONG_TYN) * LDH + k));
-#pragma unroll
-            for (int i = 0; i < LONG_RI; ++i)
-#pragma unroll
-                for (int j = 0; j < LONG_TJ; ++j) {
-                    float a = acc[i][j];
-                    a = __fmaf_rn(xv[j].x, wv[i].x, a);
-                    a = __fmaf_rn(xv[j].y, wv[i].y, a);
-                    a = __fmaf_rn(xv[j].z, wv[i].z, a);
-                    a = __fmaf_rn(xv[j].w, wv[i].w, a);
-                    acc[i][j] = a;
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < LONG_RI; ++i)
-#pragma unroll
-            for (int j = 0; j < LONG_TJ; ++j) total[i][j] = __fadd_rn(total[i][j], acc[i][j]);      // partial p joins the ordered sum
-    }
+    };
+
+    if (ranks == 1) for (uint32_t i = tid; i < RT_PART_FLOATS; i += RT_THREADS) ps[i] = 0.0f;
+    load_w(k_first, min(uint32_t(RT_CHUNK), part));
+    pdl_wait();
     pdl_launch_dependents();
-    if (narrow) {
-        const uint32_t tt = tid % LONG_TT, rr = tid / LONG_TT, e = e0 + rr, t = t0 + tt;
-        if (rr < rows_here && t < c.T) {
-            if (e < c.E) c.logits[size_t(t) * c.E + e] = c.router_bias ? __fadd_rn(total[0][0], c.router_bias[e]) : total[0][0];
-            else c.gate_logit[t] = total[0][0];
-        }
-        return;
-    }
+    load_x(k_first, min(uint32_t(RT_CHUNK), part));
+    uint64_t acc[4][TJ];                             // [row pair rg + 8 i][token tg + 16 j]
+    float single = 0.0f;
 #pragma unroll
-    for (int i = 0; i < LONG_RI; ++i) {
-        const uint32_t e = e0 + tx + LONG_TXN * i;
-        if (e >= rows_total) continue;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < LONG_TJ; ++j) {
-            const uint32_t t = t0 + ty + LONG_TYN * j;
-            if (t >= c.T) continue;
-            if (e < c.E) c.logits[size_t(t) * c.E + e] = c.router_bias ? __fadd_rn(total[i][j], c.router_bias[e]) : total[i][j];
-            else c.gate_logit[t] = total[i][j];
+        for (int j = 0; j < TJ; ++j) acc[i][j] = 0ull;
+    uint32_t in_part = 0, p = 0;                     // k done of the current partition, partitions done
+    for (uint32_t k = k_first, buf = 0; k < k_last; buf ^= 1) {
+        const uint32_t n = min(uint32_t(RT_CHUNK), part - in_part);
+        float* stage = smem + buf * RT_STAGE_FLOATS;
+        store(stage);
+        __syncthreads();                             // the chunk is in place; the other buffer's readers finished before they stored this one
+        const uint32_t next = k + n, next_in = in_part + n == part ? 0 : in_part + n;
+        if (next < k_last) { load_w(next, min(uint32_t(RT_CHUNK), part - next_in)); load_x(next, min(uint32_t(RT_CHUNK), part - next_in)); }
+        const float* ws = stage;
+        const float* xs = stage + (RT_ROWS / 2) * RT_WLD;
+        if (narrow) {
+            const uint32_t tt = tid % RT_TOKENS, rr = tid / RT_TOKENS;
+            for (uint32_t q = 0; q < n; ++q) single = __fmaf_rn(xs[tt * XLD + q], ws[q * 2 + rr], single);
+        } else {
+#pragma unroll 2
+            for (uint32_t q = 0; q < n; q += 4) {
+                ulonglong2 wv[2][4];                 // the row pairs' operands of k = q + 2 h and the next
+                float4 xv[TJ];
+#pragma unroll
+                for (int j = 0; j < TJ; ++j) xv[j] = *reinterpret_cast<const float4*>(xs + (tg + 16 * j) * XLD + q);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) wv[h][i] = *reinterpret_cast<const ulonglong2*>(ws + (rg + 8 * i) * RT_WLD + (q + 2 * h) * 2);
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)       // a chain's next link comes 4 TJ instructions later
+#pragma unroll
+                    for (int j = 0; j < TJ; ++j) {
+                        const float v = kk == 0 ? xv[j].x : kk == 1 ? xv[j].y : kk == 2 ? xv[j].z : xv[j].w;
+                        const uint64_t xd = pack2(v, v);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[i][j] = fma2(xd, kk % 2 ? wv[kk / 2][i].y : wv[kk / 2][i].x, acc[i][j]);
+                    }
+            }
+        }
+        k = next; in_part = next_in;
+        if (next_in == 0) {                          // partition p is complete
+            float* to = ps + (ranks == 1 ? 0 : p * RT_PART_FLOATS);
+            if (narrow) {
+                float* o = to + (tid % RT_TOKENS) * RT_PLD + tid / RT_TOKENS;
+                *o = ranks == 1 ? __fadd_rn(*o, single) : single;
+                single = 0.0f;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < TJ; ++j) {
+                        float2* o = reinterpret_cast<float2*>(to + (tg + 16 * j) * RT_PLD + (rg + 8 * i) * 2);
+                        const float2 v = unpack2(acc[i][j]);
+                        if (ranks == 1) { const float2 sum = *o; *o = make_float2(__fadd_rn(sum.x, v.x), __fadd_rn(sum.y, v.y)); }
+                        else *o = v;
+                        acc[i][j] = 0ull;
+                    }
+            }
+            ++p;
         }
     }
+    if (ranks == 1) __syncthreads();
+    else cg::this_cluster().sync();
+    const uint32_t share = RT_TOKENS * RT_ROWS / ranks;
+    for (uint32_t o = cr * share + tid; o < (cr + 1) * share; o += RT_THREADS) {
+        const uint32_t tt = o / RT_ROWS, el = o % RT_ROWS, t = t0 + tt, e = e0 + el;
+        if (t >= c.T || e >= rows_total) continue;
+        float sum = 0.0f;
+        if (ranks == 1) sum = ps[tt * RT_PLD + el];
+        else {
+            float v[16];
+#pragma unroll
+            for (uint32_t q = 0; q < 16; ++q) v[q] = *cg::this_cluster().map_shared_rank(ps + (q % parts) * RT_PART_FLOATS + tt * RT_PLD + el, q / parts);
+#pragma unroll
+            for (uint32_t q = 0; q < 16; ++q) sum = __fadd_rn(sum, v[q]);
+        }
+        if (e < c.E) c.logits[size_t(t) * c.E + e] = c.router_bias ? __fadd_rn(sum, c.router_bias[e]) : sum;
+        else c.gate_logit[t] = sum;
+    }
+    if (ranks > 1) cg::this_cluster().sync();        // nobody leaves while a peer may still read its partials
 }
 
-int launch_router_long(zc_moe* m, const Call& c, cudaStream_t s) {
-    if (c.router_dtype == ZC_F32 && c.act_dtype != ZC_F32 && m->router_db) {       // the double-buffered form
-        const uint32_t partd = c.H / 16;
-        const size_t bytes = 2 * (size_t(LONG_RT) * (partd + 4) * 4 + size_t(LONG_TT) * (partd + 8) * 2);
-        static SmemOptIn configured_db;
-        if (bytes <= 110 * 1024 && opt_in_smem(router_long_db_kernel, configured_db, m->device, bytes) == cudaSuccess) {
-            const uint32_t rows = c.E + (c.has_shared ? 1 : 0);
-            int rcd;
-            {
-                Timed t(m, s, KERNEL_ROUTER);
-                const cudaError_t e = launch_chained(m, -1, router_long_db_kernel, dim3((rows + LONG_RT - 1) / LONG_RT, (c.T + LONG_TT - 1) / LONG_TT), dim3(LONG_THREADS), bytes, s, nullptr, 0, c);
-                if (e != cudaSuccess) return fail(m, ZC_EEXEC, std::string("router (long, double-buffered) launch: ") + cudaGetErrorString(e));
-                rcd = check_launch(m, "router");
-            }
-            return rcd < 0 ? rcd : 1;
-        }
-        cudaGetLastError();
+template <bool X32, bool W32, int TJ>
+int launch_router_tile_n(zc_moe* m, const Call& c, uint32_t ranks, cudaStream_t s) {
+    using Tile = RouterTile<TJ>;
+    constexpr int RT_TOKENS = Tile::TOKENS, RT_STAGE_FLOATS = Tile::STAGE_FLOATS, RT_PART_FLOATS = Tile::PART_FLOATS;
+    const size_t smem = (2 * size_t(RT_STAGE_FLOATS) + size_t(ranks == 1 ? 1 : 16 / ranks) * RT_PART_FLOATS) * sizeof(float);
+    const uint32_t rows = c.E + (c.has_shared ? 1 : 0);
+    auto kernel = router_tile_kernel<X32, W32, TJ>;
+    static SmemOptIn configured;        // per instantiation, per device
+    if (opt_in_smem(kernel, configured, m->device, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    const dim3 grid(ranks, (rows + RT_ROWS - 1) / RT_ROWS, (c.T + RT_TOKENS - 1) / RT_TOKENS);
+    static int8_t usable[MAX_DEVICES];  // per device: 0 unknown, 1 the device hosts a cluster of this shape, 2 it cannot
+    if (ranks > 1 && usable[m->device] == 0) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid; cfg.blockDim = dim3(RT_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = attr; cfg.numAttrs = 1;
+        int clusters = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+        if (e != cudaSuccess) cudaGetLastError();
+        usable[m->device] = (e == cudaSuccess && clusters > 0) ? 1 : 2;
     }
-    const uint32_t part = c.H / 16, LD = part + 4;
-    const size_t smem = size_t(LONG_RT + LONG_TT) * LD * sizeof(float);
-    if (smem > 200 * 1024) return 0;
-    static SmemOptIn configured;
-    if (opt_in_smem(router_long_kernel, configured, m->device, smem) != cudaSuccess) { cudaGetLastError(); return 0; }
-    const uint32_t rows_total = c.E + (c.has_shared ? 1 : 0);
-    const dim3 grid((rows_total + LONG_RT - 1) / LONG_RT, (c.T + LONG_TT - 1) / LONG_TT);
+    if (ranks > 1 && usable[m->device] != 1) return 0;
     int rc;
     {
         Timed t(m, s, KERNEL_ROUTER);
-        const cudaError_t e = launch_chained(m, -1, router_long_kernel, grid, dim3(LONG_THREADS), smem, s, nullptr, 0, c);
-        if (e != cudaSuccess) return fail(m, ZC_EEXEC, std::string("router (long) launch: ") + cudaGetErrorString(e));
+        // Whole-K tiles are not launched early: such a CTA lives as long as the kernel, and placed while the kernel before still
+        // holds some SMs they pile up on the others (a layer of 2048 tokens: 891 us against 771). Clusters are: 602 us
+        // against 616 for the layer of 256 tokens at hidden 4096.
+        const cudaError_t e = launch_chained(m, ranks > 1 ? int(KERNEL_ROUTER) : -1, kernel, grid, dim3(RT_THREADS), smem, s, ranks > 1 ? attr : nullptr, ranks > 1 ? 1 : 0, c, ranks);
+        if (e != cudaSuccess) return fail(m, ZC_EEXEC, std::string("router (tile) launch: ") + cudaGetErrorString(e));
         rc = check_launch(m, "router");
     }
     return rc < 0 ? rc : 1;
+}
+
+template <bool X32, bool W32>
+int launch_router_tile(zc_moe* m, const Call& c, uint32_t ranks, bool wide, cudaStream_t s) {
+    return wide ? launch_router_tile_n<X32, W32, 8>(m, c, ranks, s) : launch_router_tile_n<X32, W32, 4>(m, c, ranks, s);
 }
 
 }  // namespace
 
-uint32_t router_rows_padded(const zc_moe_desc& d) { return (d.experts + (d.has_shared ? 1 : 0) + ROW_TILE_PAD - 1) / ROW_TILE_PAD * ROW_TILE_PAD; }
-
 int launch_router_partial(zc_moe* m, const Call& c, cudaStream_t s) {
-    // Cluster form for short batches, whole-K tiles for long ones (2048 tokens: 178 us against 237 us for the
-    // global-memory form; 8192: 650 against 893), the global-memory form in between (256 tokens at hidden 4096: 77 us
-    // against 205 us for 36 whole-K tiles) and whenever the device cannot host the others.
-    {
-        int n = 0;
-        // Up to 128 tokens small tiles win on latency: at 64 tokens, 544 CTAs of 16 tokens x 32 rows measured 19 us
-        // against 21 us (32 x 32) and 25 us (32 x 64, whose 144 large CTAs do not all find a cluster slot in the first wave).
-        if (c.T <= 8) n = launch_router_cluster<8, 1>(m, c, s);
-        else if (c.T <= ZC_ROUTER_SMALL_T) n = launch_router_cluster<16, 1>(m, c, s);
-        else if (size_t((c.T + 63) / 64) * ((c.E + 64) / 64) >= 144) n = launch_router_long(m, c, s);      // enough whole-K tiles to fill the SMs
+    // Up to 128 tokens small cluster tiles win on latency: at 64 tokens, 544 CTAs of 16 tokens x 32 rows measured 19 us
+    // against 21 us (32 x 32) and 25 us (32 x 64, whose 144 large CTAs do not all find a cluster slot in the first wave).
+    int n = 0;
+    if (c.T <= 8) n = launch_router_cluster<8, 1>(m, c, s);
+    else if (c.T <= ZC_ROUTER_SMALL_T) n = launch_router_cluster<16, 1>(m, c, s);
+    if (n != 0) return n;
+    // Beyond, the register-tiled form. Splitting the partitions over eight CTAs pays unless the 64 x 64 tiles fill the SMs
+    // evenly: 256 tiles (2048 tokens, 512 experts) 142 us whole against 152 us split, 376 tiles 256 against 217, 72 tiles 90
+    // against 52; from 480 tiles on, tiles of twice the tokens (a third fewer shared-memory reads per product) 387 against
+    // 405 us at 6430 tokens. A device that cannot host a cluster of eight takes whole tiles.
+    const size_t tiles = size_t((c.T + 63) / 64) * ((c.E + RT_ROWS - 1) / RT_ROWS);
+    const bool f32x = c.act_dtype == ZC_F32, f32w = c.router_dtype == ZC_F32;
+    uint32_t ranks = tiles >= 480 || (tiles >= 240 && tiles <= 296) ? 1 : CLUSTER_SIZE;
+    for (;;) {
+        n = f32x ? (f32w ? launch_router_tile<true, true>(m, c, ranks, tiles >= 480, s) : launch_router_tile<true, false>(m, c, ranks, tiles >= 480, s))
+                 : (f32w ? launch_router_tile<false, true>(m, c, ranks, tiles >= 480, s) : launch_router_tile<false, false>(m, c, ranks, tiles >= 480, s));
         if (n != 0) return n;
+        if (ranks == 1) return fail(m, ZC_EEXEC, "router: the device does not host the kernel");
+        ranks = 1;
     }
-    const uint32_t part = c.H / 16;
-    const uint32_t rows_padded = router_rows_padded(m->d);
-    // Token tile: 8 tokens x 32 rows for single-digit batches, 32 tokens x 64 rows beyond (eight chains per
-    // thread share two shared-memory reads per k); long batches use the 64-token tile, which re-reads the
-    // router rows least often.
-    const int which = c.T <= 8 ? 0 : c.T <= 512 ? 1 : 2;
-    const uint32_t TT = which == 0 ? 8 : which == 1 ? 32 : 64;
-    const uint32_t row_tile = which == 1 ? 64 : 32;
-    const size_t smem = size_t(part) * (TT + row_tile) * sizeof(float);
-    static SmemOptIn configured[3];
-    {
-        const cudaError_t e = which == 0 ? opt_in_smem(router_partial_kernel<8>, configured[0], m->device, smem)
-                            : which == 1 ? opt_in_smem(router_partial_kernel<32>, configured[1], m->device, smem)
-                                         : opt_in_smem(router_partial_kernel<64>, configured[2], m->device, smem);
-        if (e != cudaSuccess) return check_launch(m, "router attribute");
-    }
-    const uint32_t rows_total = c.E + (c.has_shared ? 1 : 0);
-    const dim3 grid((rows_total + row_tile - 1) / row_tile, 16, (c.T + TT - 1) / TT);
-    int rc;
-    {
-        Timed t(m, s, KERNEL_ROUTER);
-        if (which == 0) router_partial_kernel<8><<<grid, ROUTER_THREADS, smem, s>>>(c, m->router_partial, rows_padded, m->router_done, 1);
-        else if (which == 1) router_partial_kernel<32><<<grid, ROUTER_THREADS, smem, s>>>(c, m->router_partial, rows_padded, m->router_done, 1);
-        else router_partial_kernel<64><<<grid, ROUTER_THREADS, smem, s>>>(c, m->router_partial, rows_padded, m->router_done, 1);
-        rc = check_launch(m, "router");
-    }
-    return rc < 0 ? rc : 1;
 }
 
 // The router operator: one launch (partials, then the ordered sum by the last partition CTA of each tile).
