@@ -290,11 +290,11 @@ int zc_moe_stack_host(zc_moe* moe, const void* x_host, uint32_t tokens, void* ou
  *   0 selects the earlier per-group-drain kernel.
  *   "prefill_small_rows" (default 16, 0..64): in a long batch, experts with at most this many rows run on the streaming
  *   kernels and the grouped GEMM takes the others (0: the grouped GEMM takes every expert).
- *   "few_tiles_gate_up" (default 1), "few_tiles_down" (default 2), 1..4: 16-row tiles per warp of those streaming
- *   launches (few experts have work there: fewer tiles per warp mean more, shorter CTAs per expert).
- *   "meta_blocks" (default 1): the streaming kernels fetch scales and biases eight groups at a time (16-byte copies)
+ *   "few_tiles_gate_up" (default 1), "few_tiles_down" (default 2), 1..4: 16-row tiles per warp of the item kernels in such
+ *   launches; "meta_blocks" (default 1): the item kernels fetch scales and biases eight groups at a time (16-byte copies)
  *   for gate/up at hidden >= 4096; 2 does so wherever the layout allows, 3 uses four-group blocks for gate/up, 0 never
- *   (each ring stage's own halves, 4- or 8-byte copies). Results are identical.
+ *   (each ring stage's own halves, 4- or 8-byte copies). Both matter only where a batch runs on the item kernels (one or two
+ *   tokens, and some short batches: csrc/experts_decode.cu has the rule). Results are identical.
  *   "router_db" (0 or 1): accepted, without effect (long batches have one router form). Results are identical.
  * Changing an option drops the cached graphs of zc_moe_stack. */
 int zc_moe_set_option(zc_moe* moe, const char* name, int value);

@@ -1,0 +1,66 @@
+"""The persistent streaming expert kernels against the CPU checker, at the sizes where their cut can go wrong: K that is not
+whole stages or pairs of stages, one staged row block, warps sharing a tile, more passes per CTA than its table holds, long
+items, FP32 activations, 8-bit codes, and biases that do not follow the scales (the bias product on its own)."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+from tests import util
+from zerocool_b200 import synth
+from zerocool_b200.records import ARITH_REFERENCE, BF16, F16, F32, MoeConfig
+
+pytestmark = pytest.mark.gpu
+SEED = 11
+TOL = 2e-3          # max-abs error over the output's RMS, the specification's bound for FP32 accumulation and FP16 SwiGLU rows
+
+
+@pytest.mark.parametrize("tokens,kw", [
+    (5, dict(experts=512)),                                              # four warps per gate/up tile
+    (40, dict(hidden=4096, experts=128)),                                # one row block, four warps per tile
+    (40, dict(hidden=3072, experts=64)),
+    (33, dict(hidden=384, ffn=128, experts=32)),                         # six groups; a row of 64 code bytes
+    (70, dict(hidden=2560, ffn=640, experts=64, meta_dtype=BF16)),       # ten groups: an odd number of stages, half of the last one
+    (70, dict(hidden=1280, ffn=384, experts=64, act_dtype=F32)),         # two FP16 terms per activation, five pairs of 20 groups
+    (130, dict(hidden=512, ffn=256, experts=32)),                        # items of about forty rows
+    (5000, dict(hidden=128, ffn=128, experts=32, top_k=8, act_dtype=F32)),   # 5,600 passes: more than a table of 32 per CTA
+    (45, dict(hidden=2048, experts=64, down_bits=8, q8_signed=1)),
+    (45, dict(hidden=640, ffn=128, experts=32, gate_bits=8, up_bits=8, down_bits=8)),
+    (30, dict(hidden=2048, experts=64, gate_bits=8, up_bits=8, down_bits=4)),
+    (64, dict(hidden=2560, ffn=640, experts=64, meta_dtype=BF16, act_dtype=F32, router_dtype=BF16, arith=ARITH_REFERENCE)),
+])
+def test_streamed_experts_against_the_checker(tokens, kw):
+    torch = pytest.importorskip("torch")
+    from zerocool_b200.moe import Moe
+    base = dict(hidden=2048, ffn=512, experts=64, top_k=10, layers=1, meta_dtype=F16, act_dtype=BF16, out_dtype=F32, router_dtype=F32, has_shared=1, max_tokens=tokens)
+    base.update(kw)
+    cfg = MoeConfig(**base)
+    rng = np.random.default_rng(tokens)
+    records = [util.asymmetric_record(cfg, SEED, 0, e, rng) for e in range(cfg.experts)]
+    shared = util.asymmetric_record(cfg, SEED, 0, synth.SHARED_EXPERT, rng)
+    m = Moe(cfg, 0)
+    w, gate = synth.router(cfg, SEED, 0), synth.shared_gate(cfg, SEED, 0)
+    m.load_layer(0, np.stack(records), router_w=w, shared_record=shared, shared_gate_w=gate)
+    x = synth.activations(cfg, SEED, 0, tokens)
+    if cfg.gate_bits > cfg.down_bits:
+        x = x / 16          # the generator's 8-bit weights reach 2.5: keeps the SwiGLU rows inside the 4-bit down projection's range (4094)
+    dev = torch.from_numpy(x).to(device="cuda", dtype=m.act_torch)
+    got = m.decode(0, dev)
+    assert m.status() == 0
+    ids = m.last_routing(tokens)["ids"]
+    want = oracle.moe_layer(cfg.as_dict(), records, w, x, shared_record=shared, shared_gate_w=gate)
+    assert np.array_equal(ids, want["ids"])
+    err = util.rel_max_error(got.cpu().numpy(), want["out"])
+    # The reference arithmetic rounds to BF16 at every boundary: one step (2^-8 of a value of a few RMS) where a sum lies on one.
+    assert err <= (0.05 if cfg.arith == ARITH_REFERENCE else TOL), err
+    assert torch.equal(m.decode(0, dev), got)
+
+
+def test_a_token_does_not_depend_on_its_place_in_the_batch():
+    torch = pytest.importorskip("torch")
+    from zerocool_b200.moe import Moe
+    cfg = util.cfg2(experts=64, max_tokens=200)
+    m = Moe(cfg, 0)
+    m.synth_fill_layer(0, SEED)
+    x = torch.from_numpy(synth.activations(cfg, SEED, 0, 200)).to(device="cuda", dtype=torch.bfloat16)
+    order = torch.from_numpy(np.random.default_rng(3).permutation(200)).cuda()
+    assert torch.equal(m.decode(0, x)[order], m.decode(0, x[order].contiguous()))

@@ -1,5 +1,6 @@
 // Shared device helpers and the handle layout of the B200 MoE library.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -82,6 +83,7 @@ inline uint64_t record_bytes_of(const zc_moe_desc& d) {
 // ---------------------------------------------------------------------------------------------
 // Handle
 // ---------------------------------------------------------------------------------------------
+struct StreamMap { CUtensorMap m; };
 struct LayerMem {
     uint8_t* records = nullptr;       // [local_experts, record_stride]
     void* router_w = nullptr;         // [E, H]
@@ -89,6 +91,8 @@ struct LayerMem {
     void* shared_gate_w = nullptr;    // [1, H], or null
     float* router_bias = nullptr;     // [E] added to the logits after the partition sum; storage always present
     bool bias_set = false;
+    // TMA views of the records' codes for the streaming kernels (experts_decode.cu)
+    StreamMap map_gate_up, map_down, map_shared_gate_up, map_shared_down;
 };
 
 // Everything a kernel needs to know about one call, passed by value.
@@ -271,6 +275,7 @@ struct zc_moe {
     uint32_t prefill_small_rows = 16;   // long batches: experts with at most this many rows run on the streaming kernels (0 = none)
     bool prefill_wide = true;     // long batches: wide-tile kernel with accumulators resident in TMEM (false: per-group drain kernel)
     bool fold_q4 = true;          // Q4 codes enter the MMA with their 1024 offset (removed from the FP32 group sum)
+    bool stream_maps = true;      // the records' geometry has TMA views (make_stream_maps)
     bool profiling = false;
     struct Span { int kind; cudaEvent_t start, stop; };
     std::vector<Span> spans;
@@ -283,6 +288,8 @@ int launch_router_partial(zc_moe* m, const Call& c, cudaStream_t s);
 int launch_route_permute(zc_moe* m, const Call& c, cudaStream_t s, bool do_route, bool do_permute);
 int launch_forced_weights(zc_moe* m, const Call& c, const int32_t* forced, cudaStream_t s);
 int launch_experts_decode(zc_moe* m, const Call& c, cudaStream_t s);
+int launch_experts_item(zc_moe* m, const Call& c, cudaStream_t s);           // one CTA per (item, row tiles): experts_item.cu
+int make_stream_maps(zc_moe* m, LayerMem& L);                                // TMA views of a layer's records (experts_decode.cu)
 int launch_experts_prefill(zc_moe* m, const Call& c, cudaStream_t s, uint32_t skip_rows_upto = 0);
 bool prefill_supported(const zc_moe_desc& d);
 size_t prefill_tile_capacity(const zc_moe_desc& d);

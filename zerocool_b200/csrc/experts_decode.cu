@@ -9,80 +9,73 @@
 //   NMAT = 2 (gate/up): h[row, f]  = silu(gate_e . x_row) * (up_e . x_row)    for every (expert, row)
 //   NMAT = 1 (down):    y[slot, c] = down_e . h_row, written at the slot's router position
 //
-// Each launch streams every selected record once per eight rows. At B200 rates the limiting resource
-// is instruction issue, not arithmetic: 4-bit codes arrive at ~13 T weights/s, about three issue slots
-// per weight per SM. So:
+// Each launch streams every selected record once per eight rows (a pass). What bounds it is HBM as long as a weight costs few
+// enough instructions: at 6.5 TB/s an SM receives ~46 4-bit weights per clock and can issue four warp instructions, so 1,024
+// weights (16 rows x 64 k, one quantisation group of a tile) have ~88 issue slots at best. The item kernels spend 82
+// instructions on them (ncu), this one 57, 36 of which are the product itself; in mid-launch a warp's 1,024 weights take
+// 23.4 clocks of its SM, against 22 at the copy bandwidth. Layers measured against the item kernels (us): 5 tokens 58 -> 49,
+// 64 tokens 176 -> 170, 160 tokens 254 -> 231, 400 tokens 405 -> 349, 256 tokens at hidden 4096 605 -> 492; 700 tokens with
+// Zipf-skewed loads 1816 -> 438 (the passes of one long item are spread over the machine instead of two CTAs).
+// What is left at 64 tokens: ~8 us per launch until the first product (item list, tables, rows, then the first 128 KB per SM),
+// and ends of the CTAs' runs that differ by up to a tenth.
 //  * The multiply-accumulates run on the tensor cores as m16n8k16 FP16 MMAs with up to eight token
-//    rows in the N dimension. Integer codes are exact in FP16, a BF16 activation converts exactly, an
-//    FP32 activation is split into two FP16 terms, and products are accumulated in FP32 per 64-wide
-//    quantisation group. The group's scale and bias are applied to that FP32 accumulator:
-//        acc += scale[row, g] * sum_k(q * x) + bias[row, g] * sum_k(x)
-//    which is the reference's affine_dot form (qwen.metal:46-62) with an exact inner sum.
+//    rows in the N dimension. Integer codes are exact in
+//    FP16, a BF16 activation converts exactly, an FP32 activation is split into two FP16 terms, and products are
+//    accumulated in FP32 per 64-wide quantisation group. The group's scale is applied to that FP32 sum; the bias term is
+//    a product of its own:
+//        acc += scale[row, g] * sum_k(q * x);     acc += bias[row, :] . group sums of x
+//    which is the reference's affine_dot form (qwen.metal:46-62) with an exact inner sum. The bias product is an
+//    m16n8k4 TF32 MMA over four groups: a 16-bit bias is exact in TF32, and the FP32 group sum enters as two TF32 terms
+//    (22 significant bits), so it replaces two conversions and four FMAs per group and 16 x 8 tile by a fraction of an MMA.
 //  * Q4 codes become FP16 with one logic operation per two weights: (w & 0x000f000f) | 0x6400 is the
 //    half2 (1024+q_lo, 1024+q_hi), and (w & 0x00f000f0) | 0x6400 is (1024+16 q, 1024+16 q). With FOLD
 //    those values go into the MMA as they are: the activations that meet a "q" slot are staged multiplied by 16
-//    (exact; the finished sum is divided by 16), and the 1024 offset is removed from the FP32 group sum as
-//    1024 * sum(x as staged).
+//    (exact; the finished sum is divided by 16), and the 1024 offset is removed from the FP32 group sum, which starts
+//    from -1024 * sum(x as staged).
 //    Without FOLD the offset and the factor 16 are removed in FP16 before the MMA (exact, 4 more ops per
 //    word).
-//  * Weights reach the warp through a private cp.async ring in shared memory (no registers held
-//    across the latency, no block-wide barrier). A stage holds CH quantisation groups of a 16-row tile:
-//    each row's CH * 32 (Q4) or CH * 64 (Q8) contiguous code bytes are fetched as 16-byte pieces by
-//    adjacent lanes, so every sector of a record is requested once; the 32/64-byte blocks of a row are
-//    XOR-swizzled by the row index so that the fragment reads stay bank-conflict free. The refill of a
-//    slot is issued before the chunk that was waited for is multiplied, so STAGES-1 chunks are in
-//    flight while the warp computes.
-//  * Lanes whose token row is absent (fewer than eight rows in the pass) skip the activation reads.
+//  * Codes reach a warp through its own ring of two 4 KB stages, filled by one TMA instruction per stage (a box of 32 rows
+//    x 128 bytes: 16 rows of gate and of up, or 32 rows of down), so a copy costs no address arithmetic and no L1. The
+//    128-byte swizzle exchanges 16-byte pieces by row mod 8; MMA row g reads tile row pi(g) = 0,4,2,6,1,5,3,7, with which
+//    the 8-byte (Q4) and 16-byte (Q8) fragment reads of a warp hit every bank once.
+//  * Scales and biases are read straight from global memory into registers, one stage ahead: the four lanes of a row share
+//    an 8-byte read of four scales, and each lane fetches the one bias it supplies to the bias product.
+//  * The grid is one persistent CTA per SM. The passes of all items are laid end to end (a block-wide scan of the
+//    permutation's item list, which every CTA does for itself), every pass is cut into units of RT row tiles, and CTA b
+//    takes the b-th of gridDim.x equal runs of units: no last wave, and the copies of the next unit are in flight while a
+//    unit is finished. KS warps share a row tile by taking every KS-th stage of K; their partial sums are added in warp
+//    order by one of them (a different one for each unit).
+//  * Lanes whose token row is absent skip the activation reads.
 //  * Because a dot product does not care about the order of k, the MMA's k slots are bound to whatever
 //    k values fall out of the cheapest extraction; the activations are staged in the matching order.
 // Activations must stay inside FP16 after the factor 16 (|x| < 4094 for Q4 projections, < 65504 for Q8); hidden
 // states after a norm are O(1..100). A value beyond that raises ZC_STATUS_RANGE in the status word (the output of
 // that row is then not meaningful); the same holds for the SwiGLU rows the down projection reads.
+#include <cmath>
+
 #include "common.cuh"
 
 namespace zc {
 namespace {
 
-constexpr int NTOK = 8;               // token rows per MMA pass (the N of m16n8k16)
-constexpr int WARPS = 8;
-constexpr int EXPERT_THREADS = WARPS * 32;
+constexpr int NROW = 8;               // token rows of a pass (the N of m16n8k16)
+constexpr int MAX_WARPS = 16;
+constexpr int MAX_THREADS = MAX_WARPS * 32;
 constexpr int ROW_PAD = 8;            // halves added to each staged row (keeps 16-byte reads conflict free)
-#ifndef ZC_MIN_BLOCKS
-#define ZC_MIN_BLOCKS 2
-#endif
-#ifndef ZC_MIN_BLOCKS_DOWN
-#define ZC_MIN_BLOCKS_DOWN 3
-#endif
-
-// One ring stage of one matrix holds CHT quantisation groups of 16 rows: for every row one LINE of CHT x ROWB
-// contiguous code bytes (a full 128-byte line for Q4 with four groups and for Q8 with two).
-template <int BITS, int CHT> struct Fmt {
-    static constexpr int ROWB = BITS * 8;                 // code bytes of one row of one group (64 weights)
-    static constexpr int LINE = CHT * ROWB;               // code bytes of one row in one stage
-    static constexpr int PIECES = LINE / 16;              // 16-byte pieces (= lanes) per row
-    static constexpr int ROWS_PER_PASS = 32 / PIECES;
-    static constexpr int PASSES = 16 / ROWS_PER_PASS;
-    static constexpr int CODES = 16 * LINE;
-    static constexpr int MATRIX = CODES;                  // a ring stage holds the codes only
-    // Metadata of a matrix, beside the ring: [buffer][row][scale, bias][MG halves]. MG = 8 groups per block (one 16-byte
-    // copy per (row, kind), two buffers) where a warp walks K in order, else MG = CHT (one block per ring stage).
-    __host__ __device__ static constexpr int meta_area(int mbg, int stages) { return mbg ? 2 * 32 * mbg * 2 : stages * 32 * CHT * 2; }     // bytes per matrix per warp (mbg: groups per block, 0 = per stage)
-    // Rows whose lines fall into the same 128-byte bank window are ROWS_PER_WINDOW apart; the block index of a row is
-    // xor-ed with swizzle(row) so that rows read together by one MMA fragment load use different banks.
-    static constexpr int ROWS_PER_WINDOW = LINE >= 128 ? 1 : 128 / LINE;
-    __host__ __device__ static constexpr uint32_t swizzle(uint32_t row) { return (row / ROWS_PER_WINDOW) & (CHT - 1); }
-};
+constexpr int STAGES = 2;             // ring stages per warp
+constexpr int STAGE_BYTES = 4096;     // 32 rows x 128 code bytes
+constexpr int TABLE = 32;             // passes whose descriptors and rows a CTA keeps at a time
+constexpr uint32_t PERM_CACHE = 1024;  // a permutation up to this long is fetched whole while the item list is read
+constexpr uint32_t POLL_LIMIT = 1u << 18;     // attempts of a bounded wait, each suspended for at most about a microsecond
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // D(16x8, fp32) += A(16x16, fp16, row) * B(16x8, fp16, col). Lane (g = lane/4, c = lane%4) holds
 //   a0: A[g][2c,2c+1]   a1: A[g+8][2c,2c+1]   a2: A[g][2c+8,2c+9]   a3: A[g+8][2c+8,2c+9]
 //   b0: B[2c,2c+1][g]   b1: B[2c+8,2c+9][g]
 //   d0,d1: D[g][2c,2c+1]   d2,d3: D[g+8][2c,2c+1]
 __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -90,168 +83,151 @@ __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32
 // Same product with the addend taken from c (the first MMA of a group starts from the folded offset).
 __device__ __forceinline__ void mma_f16_16816_c(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
                                                 float c0, float c1, float c2, float c3) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 
-// Ring depth per warp: two stages of four groups or three of two keep the same bytes in flight.
-__host__ __device__ constexpr int stages_for(int matrices_per_warp, int ch) { return (ch == 4 && matrices_per_warp == 2) ? 2 : 3; }
-
-struct ItemInfo {
-    const uint8_t* record;
-    uint32_t count;     // rows of this item
-    uint32_t pos0;      // routed: first position in perm; shared: first token of this block of rows
-    uint32_t hrow0;     // first row in hbuf
-    bool shared;
-};
-
-// Items of a launch: the shared expert contributes one item per NTOK tokens (so that its row blocks run
-// in parallel instead of as passes of one CTA), then one item per routed expert that received work.
-__device__ __forceinline__ bool decode_item(const Call& c, uint32_t item, ItemInfo& it) {
-    if (c.has_shared) {
-        const uint32_t blocks = (c.T + NTOK - 1) / NTOK;
-        if (item < blocks) {
-            it.record = c.shared_record; it.pos0 = item * NTOK; it.count = min(uint32_t(NTOK), c.T - it.pos0);
-            it.hrow0 = c.T * c.K + it.pos0; it.shared = true;
-            return true;
-        }
-        item -= blocks;
-    }
-    const int4 entry = __ldcg(c.items + item);            // one load: {expert, first position, rows}; x = -1 past the list's end
-    if (entry.x < 0) return false;
-    if (c.item_rows_max && uint32_t(entry.z) > c.item_rows_max) return false;      // this expert's rows go to the tensor-core family
-    const uint32_t e = uint32_t(entry.x);
-    it.record = c.records + size_t(e - c.first_expert) * c.record_stride;
-    it.pos0 = uint32_t(entry.y);
-    it.count = uint32_t(entry.z);
-    it.hrow0 = it.pos0;
-    it.shared = false;
-    return true;
+// D(16x8, fp32) += A(16x4, tf32) * B(4x8, tf32): a0: A[g][c], a1: A[g+8][c], b0: B[c][g].
+__device__ __forceinline__ void mma_tf32_1684(float (&d)[4], float a0, float a1, float b0) {
+    asm("mma.sync.aligned.m16n8k4.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(b0)));
 }
 
-// Stage the valid source rows (n < nvalid) of K elements into shared memory as FP16 (hi, and lo when
+// D(16x8, fp32) += A(16x8, tf32) * B(8x8, tf32): a0: A[g][c], a1: A[g+8][c], a2: A[g][c+4], a3: A[g+8][c+4], b0: B[c][g], b1: B[c+4][g].
+__device__ __forceinline__ void mma_tf32_1688(float (&d)[4], float a0, float a1, float a2, float a3, float b0, float b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+
+// How a launch is cut (chosen on the host, stream_plan): warps per CTA, warps that share a row tile, staged passes,
+// and what follows from them.
+struct StreamPlan {
+    uint32_t warps, ks, nbuf;
+    uint32_t rt, ks_shift;           // warps / ks; log2(ks)
+    uint32_t tiles_per_pass;         // row tiles of one pass: N / TILE
+    uint32_t pairs;                  // stage pairs of a row's K, the last one padded
+    uint32_t own;                    // item-list entries per thread
+    float inv_tiles, inv_grid;
+};
+
+// The TMA view of one projection (pair) of all records: [expert][matrix][row][byte], and the same of the shared record.
+struct StreamMaps { CUtensorMap routed, shared; };
+
+__device__ __forceinline__ void ring_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int row, int expert) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(STAGE_BYTES) : "memory");
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(row), "r"(0), "r"(expert), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void group_sync(uint32_t id, uint32_t threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void group_arrive(uint32_t id, uint32_t threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// n / d by a reciprocal and one correction (quotients below 2^20: the estimate is off by one at most).
+__device__ __forceinline__ uint32_t quick_div(uint32_t n, uint32_t d, float inverse) {
+    uint32_t q = __float2uint_rz(__uint2float_rn(n) * inverse);
+    const int r = int(n - q * d);
+    if (r < 0) --q;
+    else if (uint32_t(r) >= d) ++q;
+    return q;
+}
+
+__device__ __forceinline__ void bar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+
+// Stage this warp's share of the valid source rows (n < nvalid) of K elements into shared memory as FP16 (hi, and lo when
 // SPLIT), in the k order the MMA fragments expect, with the per-group sums
-//   sums[grp][n] = (Sx, P):  Sx = sum of x over the group (REF: the reference's BF16 sum of four,
-//   qwen.metal:55), P = -1024 * sum of the values as staged: the MMA accumulator starts from P, which
-//   removes the folded 1024 offset of the codes (0 without FOLD).
+//   sx[n][grp] = sum of x over the group (REF: the reference's BF16 sum of four, qwen.metal:55), times 16 when FOLD;
+//   offs[grp][n / 2][4] = -1024 * sum of the values as staged (0 without FOLD), laid out as the four accumulators of a
+//   lane: the MMA starts from it, which removes the folded 1024 offset of the codes.
 //   Q4 order inside each block of 8: (0,4,1,5,2,6,3,7), even k staged x 16 when FOLD; Q8: natural order.
 // Rows n >= nvalid are left as they are: an MMA column only depends on its own B column.
-template <bool Q4ORDER, bool SPLIT, bool FOLD>
-__device__ __forceinline__ void stage_rows(const void* src, bool src_f32, const int* rows, uint32_t nvalid,
-                                           uint32_t K, bool ref, __half* hi, __half* lo, float* sums, uint32_t* status) {
-    const uint32_t RS = K + ROW_PAD, blocks = K / 8, total = nvalid * blocks;
-    bool out_of_range = false;
-    // The trip count is uniform per warp (the shuffles below need all 32 lanes); lanes past the end carry zeros.
-    for (uint32_t idx = threadIdx.x; (idx & ~31u) < total; idx += EXPERT_THREADS) {
-        const bool live = idx < total;
-        const uint32_t n = live ? idx / blocks : 0, q = live ? idx % blocks : 0;
-        const int row = rows[n];
+// A warp takes 256 consecutive elements of a row at a time (eight per lane), pieces `first`, `first + stride`, ...
+template <bool Q4ORDER, bool SPLIT, bool FOLD, typename RowOf>
+__device__ __forceinline__ void stage_rows(const void* src, bool src_f32, RowOf row_of, uint32_t nvalid, uint32_t K, uint32_t RS, uint32_t GP,
+                                           bool ref, __half* hi, __half* lo, float* sx_out, float* offs, uint32_t* status, uint32_t first, uint32_t stride) {
+    const uint32_t per_row = (K + 255) / 256, lane = threadIdx.x % 32;
+    float most = 0.0f;
+    uint32_t n = 0, piece = first;
+    while (n < nvalid) {
+        while (piece >= per_row) { piece -= per_row; ++n; }
+        if (n >= nvalid) break;
+        const uint32_t q = piece * 32 + lane;
+        const bool live = q * 8 < K;           // a row's last piece may be short; its idle lanes carry zeros through the shuffles
+        const size_t row = row_of(n);
         float v[8];
         if (!live) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = 0.0f;
         } else if (src_f32) {
-            const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(src) + size_t(row) * K + q * 8);
-            const float4 a = p[0], b = p[1];
+            const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(src) + row * K + q * 8);
+            const float4 a = __ldcg(p), b = __ldcg(p + 1);
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
         } else {
-            const uint4 raw = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(src) + size_t(row) * K + q * 8);
+            const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(src) + row * K + q * 8));
             const uint32_t r[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(r[i] << 16); v[2 * i + 1] = __uint_as_float(r[i] & 0xffff0000u); }
         }
-        float sx;
+        float sx = 0.0f;
         if (ref) sx = bf_round(bf_round(bf_round(v[0] + v[1]) + v[2]) + v[3]) + bf_round(bf_round(bf_round(v[4] + v[5]) + v[6]) + v[7]);
-        else sx = (((v[0] + v[1]) + v[2]) + v[3]) + (((v[4] + v[5]) + v[6]) + v[7]);
-        __half h[8], l[8];
-        float sf = 0.0f, sn = 0.0f;        // sums of the values as fed to the MMA: as staged, and in natural scale
+        // folded Q4 codes: the value that meets a "1024 + 16 q" slot must be 1/16 of its neighbours'. Even slots are
+        // staged x 16 rather than odd slots / 16, which keeps small activations out of FP16's subnormal range; the
+        // accumulated result is multiplied by 1/16 (exact) when it is finished.
+        constexpr float EVEN = (FOLD && Q4ORDER) ? 16.0f : 1.0f;
+        constexpr int order_q4[8] = {0, 4, 1, 5, 2, 6, 3, 7};
+        uint32_t ph[4], pl[4];
+        float even = 0.0f, odd = 0.0f;         // sums of the values as fed to the MMA
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            // folded Q4 codes: the value that meets a "1024 + 16 q" slot must be 1/16 of its neighbours'. Even slots are
-            // staged x 16 rather than odd slots / 16, which keeps small activations out of FP16's subnormal range; the
-            // accumulated result is multiplied by 1/16 (exact) when it is finished.
-            const float pre = (FOLD && Q4ORDER && !(i & 1)) ? v[i] * 16.0f : v[i];
-            out_of_range |= fabsf(pre) > 65504.0f;          // would become an FP16 infinity: reported, not hidden
-            h[i] = __float2half_rn(pre);
-            float fed = __half2float(h[i]);
-            if (SPLIT) { l[i] = __float2half_rn(pre - fed); fed += __half2float(l[i]); }
-            sf += fed;
-            sn += (FOLD && Q4ORDER && !(i & 1)) ? fed * 0.0625f : fed;
+        for (int i = 0; i < 4; ++i) {
+            const int a = Q4ORDER ? order_q4[2 * i] : 2 * i, b = Q4ORDER ? order_q4[2 * i + 1] : 2 * i + 1;
+            const float va = (a & 1) ? v[a] : v[a] * EVEN, vb = (b & 1) ? v[b] : v[b] * EVEN;
+            most = fmaxf(most, fmaxf(fabsf(va), fabsf(vb)));
+            const __half2 h = __floats2half2_rn(va, vb);
+            ph[i] = *reinterpret_cast<const uint32_t*>(&h);
+            float2 fed = __half22float2(h);
+            if (SPLIT) {
+                const __half2 l = __floats2half2_rn(va - fed.x, vb - fed.y);
+                pl[i] = *reinterpret_cast<const uint32_t*>(&l);
+                const float2 low = __half22float2(l);
+                fed.x += low.x; fed.y += low.y;
+            }
+            if (a & 1) odd += fed.x; else even += fed.x;
+            if (b & 1) odd += fed.y; else even += fed.y;
         }
         // The bias term multiplies the sum of the activations. Outside the reference arithmetic it uses the sum of
         // the values the MMA really sees, so that a rounding of an activation to FP16 enters the result through the
         // weight s q + b and not through s q alone.
-        if (!ref) sx = sn;
+        if (!ref) sx = even * (1.0f / EVEN) + odd;
+        float sf = even + odd;
 #pragma unroll
         for (int off = 1; off <= 4; off <<= 1) {
             sx += __shfl_xor_sync(0xffffffffu, sx, off);
-            sf += __shfl_xor_sync(0xffffffffu, sf, off);
+            if (FOLD) sf += __shfl_xor_sync(0xffffffffu, sf, off);
         }
-        if (!live) continue;
-        if ((q & 7) == 0) *reinterpret_cast<float2*>(sums + ((q / 8) * NTOK + n) * 2) = make_float2((FOLD && Q4ORDER) ? 16.0f * sx : sx, FOLD ? -1024.0f * sf : 0.0f);
-        constexpr int order_q4[8] = {0, 4, 1, 5, 2, 6, 3, 7};
-        uint32_t ph[4], pl[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int a = Q4ORDER ? order_q4[2 * i] : 2 * i, b = Q4ORDER ? order_q4[2 * i + 1] : 2 * i + 1;
-            ph[i] = uint32_t(__half_as_ushort(h[a])) | (uint32_t(__half_as_ushort(h[b])) << 16);
-            if (SPLIT) pl[i] = uint32_t(__half_as_ushort(l[a])) | (uint32_t(__half_as_ushort(l[b])) << 16);
+        if (live) {
+            if ((lane & 7) == 0) {
+                sx_out[n * GP + q / 8] = (FOLD && Q4ORDER) ? 16.0f * sx : sx;
+                if (FOLD) {                    // the MMA's addend of a lane: {tokens 2c, 2c + 1} for row g, the same for row g + 8
+                    float* o = offs + (q / 8) * (2 * NROW) + (n / 2) * 4 + n % 2;
+                    o[0] = o[2] = -1024.0f * sf;
+                }
+            }
+            *reinterpret_cast<uint4*>(hi + n * RS + q * 8) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+            if (SPLIT) *reinterpret_cast<uint4*>(lo + n * RS + q * 8) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
         }
-        *reinterpret_cast<uint4*>(hi + n * RS + q * 8) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-        if (SPLIT) *reinterpret_cast<uint4*>(lo + n * RS + q * 8) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+        piece += stride;
     }
-    if (out_of_range) atomicOr(status, ZC_STATUS_RANGE);
-}
-
-// Source of one matrix for this lane's cp.async copies. A pass of the warp copies ROWS_PER_PASS rows: the
-// PIECES lanes of a row fetch its LINE as one contiguous run (one 128-byte request per row where the line is
-// 128 bytes, instead of one request per 32-byte sector). In shared memory a row's groups are stored with
-// the group index xor-ed by Fmt::swizzle(row), which keeps the MMA's row-strided reads free of bank conflicts.
-template <int BITS, int CHT>
-struct LaneSource {
-    using F = Fmt<BITS, CHT>;
-    const uint8_t* codes;      // record + codes offset + (row in pass) * row_bytes + piece * 16
-    const uint8_t* meta;       // record + scales or biases offset (by kind) + row * G * 2
-    uint32_t row_bytes, dst0, meta_pair;      // meta_pair: this lane's (row, kind) index in a metadata block
-    const uint8_t* tile_codes; // set per tile
-    const uint8_t* tile_meta;
-    __device__ __forceinline__ void init(const uint8_t* record, const Projection& pr, uint32_t lane, uint32_t G) {
-        row_bytes = pr.K * BITS / 8;
-        const uint32_t piece = lane % F::PIECES, rip = lane / F::PIECES;
-        const uint32_t block = piece * 16 / F::ROWB, within = piece * 16 % F::ROWB;
-        dst0 = rip * F::LINE + ((block ^ F::swizzle(rip)) * F::ROWB) + within;      // swizzle(rip) == swizzle(row): passes add multiples of 4 rows
-        codes = record + pr.codes + size_t(rip) * row_bytes + piece * 16;
-        meta = record + (lane / 16 ? pr.biases : pr.scales) + size_t(lane % 16) * G * 2;
-        meta_pair = (lane % 16) * 2 + lane / 16;
-    }
-    __device__ __forceinline__ void set_tile(uint32_t row0, uint32_t G) {
-        tile_codes = codes + size_t(row0) * row_bytes;
-        tile_meta = meta + size_t(row0) * G * 2;
-    }
-};
-
-// Issue the cp.async copies of one chunk (CHT groups starting at grp0) of one matrix into a ring stage, and the
-// metadata that goes with it. MB8: one 16-byte copy per (row, kind) every eight groups, into buffer meta_buf of two (a
-// 4-byte copy per chunk moves a whole 32-byte sector for it and costs as many shared-memory wavefronts as a code copy);
-// otherwise the chunk's own scale and bias halves, into the buffer of its ring slot.
-template <int BITS, int CHT, int MBG>
-__device__ __forceinline__ void issue_matrix(uint32_t stage, uint32_t meta_area, const LaneSource<BITS, CHT>& src, uint32_t grp0, uint32_t meta_buf, bool meta_now) {
-    using F = Fmt<BITS, CHT>;
-    const uint8_t* g0 = src.tile_codes + grp0 * F::ROWB;
-#pragma unroll
-    for (int p = 0; p < F::PASSES; ++p)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(stage + src.dst0 + p * F::ROWS_PER_PASS * F::LINE),
-                     "l"(g0 + size_t(p * F::ROWS_PER_PASS) * src.row_bytes) : "memory");
-    if constexpr (MBG == 8) {
-        if (meta_now) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(meta_area + meta_buf * 512 + src.meta_pair * 16), "l"(src.tile_meta + grp0 * 2) : "memory");
-    } else if constexpr (MBG == 4) {
-        if (meta_now) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(meta_area + meta_buf * 256 + src.meta_pair * 8), "l"(src.tile_meta + grp0 * 2) : "memory");
-    } else if constexpr (CHT == 4) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(meta_area + meta_buf * (32 * CHT * 2) + src.meta_pair * CHT * 2), "l"(src.tile_meta + grp0 * 2) : "memory");
-    } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(meta_area + meta_buf * (32 * CHT * 2) + src.meta_pair * CHT * 2), "l"(src.tile_meta + grp0 * 2) : "memory");
-    }
+    if (!(most <= 65504.0f)) atomicOr(status, ZC_STATUS_RANGE);        // would become an FP16 infinity: reported, not hidden
 }
 
 // (a & b) | c in one logic instruction.
@@ -292,343 +268,541 @@ __device__ __forceinline__ void dequant_q8(uint32_t w, bool is_signed, uint32_t 
     p[1] = *reinterpret_cast<const uint32_t*>(&b);
 }
 
-// d(16 rows x 8 tokens) = sum over one 64-wide group of code * x for the lane's rows g (w0) and g+8 (w1).
+// d[m] (16 rows x 8 tokens) = off + sum over one 64-wide group of code * x, for the two 16-row fragments m of a stage (the
+// lane's rows g: w[m][0], g+8: w[m][1]). The fragments' independent MMA chains are interleaved.
 template <int BITS, bool SPLIT, bool FOLD>
-__device__ __forceinline__ void group_mma(float (&d)[4], float c0, float c1, const uint32_t* w0, const uint32_t* w1, const uint4 (&bh)[2], const uint4 (&bl)[2], bool q8_signed) {
-    if constexpr (BITS == 4) {
+__device__ __forceinline__ void group_mma(float (&d)[2][4], const float4& off, const uint32_t (&w)[2][2][BITS / 2],
+                                          const uint4 (&bh)[2], const uint4 (&bl)[2], bool q8_signed) {
+    constexpr int PER = BITS == 4 ? 2 : 1, STEPS = BITS == 4 ? 2 : 4;      // MMAs per code word, code words
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            uint32_t p0[4], p1[4];
-            dequant_q4<FOLD>(w0[m], p0);
-            dequant_q4<FOLD>(w1[m], p1);
-            if (m == 0) mma_f16_16816_c(d, p0[0], p1[0], p0[1], p1[1], bh[m].x, bh[m].y, c0, c1, c0, c1);
-            else mma_f16_16816(d, p0[0], p1[0], p0[1], p1[1], bh[m].x, bh[m].y);
-            mma_f16_16816(d, p0[2], p1[2], p0[3], p1[3], bh[m].z, bh[m].w);
-            if constexpr (SPLIT) {
-                mma_f16_16816(d, p0[0], p1[0], p0[1], p1[1], bl[m].x, bl[m].y);
-                mma_f16_16816(d, p0[2], p1[2], p0[3], p1[3], bl[m].z, bl[m].w);
+    for (int i = 0; i < STEPS; ++i) {
+        uint32_t p[2][2][2 * PER];
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                if constexpr (BITS == 4) dequant_q4<FOLD>(w[m][r][i], p[m][r]);
+                else dequant_q8(w[m][r][i], q8_signed, p[m][r]);
             }
-        }
-    } else {
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            uint32_t p0[2], p1[2];
-            dequant_q8(w0[m], q8_signed, p0);
-            dequant_q8(w1[m], q8_signed, p1);
-            const uint32_t b0 = (m & 1) ? bh[m / 2].z : bh[m / 2].x, b1 = (m & 1) ? bh[m / 2].w : bh[m / 2].y;
-            if (m == 0) mma_f16_16816_c(d, p0[0], p1[0], p0[1], p1[1], b0, b1, c0, c1, c0, c1);
-            else mma_f16_16816(d, p0[0], p1[0], p0[1], p1[1], b0, b1);
-            if constexpr (SPLIT) {
-                const uint32_t c0 = (m & 1) ? bl[m / 2].z : bl[m / 2].x, c1 = (m & 1) ? bl[m / 2].w : bl[m / 2].y;
-                mma_f16_16816(d, p0[0], p1[0], p0[1], p1[1], c0, c1);
+        for (int h = 0; h < PER; ++h) {
+            const int step = i * PER + h;                                  // of the group's four
+            const uint4 hi = bh[step / 2], lo = bl[step / 2];
+            const uint32_t b0 = step % 2 ? hi.z : hi.x, b1 = step % 2 ? hi.w : hi.y;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                if (step == 0) mma_f16_16816_c(d[m], p[m][0][0], p[m][1][0], p[m][0][1], p[m][1][1], b0, b1, off.x, off.y, off.z, off.w);
+                else mma_f16_16816(d[m], p[m][0][2 * h], p[m][1][2 * h], p[m][0][2 * h + 1], p[m][1][2 * h + 1], b0, b1);
+                if constexpr (SPLIT)
+                    mma_f16_16816(d[m], p[m][0][2 * h], p[m][1][2 * h], p[m][0][2 * h + 1], p[m][1][2 * h + 1], step % 2 ? lo.z : lo.x, step % 2 ? lo.w : lo.y);
             }
         }
     }
 }
 
+// Two 16-bit metadata values of a word as FP32.
+template <bool META_F16>
+__device__ __forceinline__ float2 meta_pair(uint32_t w) {
+    if constexpr (META_F16) return __half22float2(*reinterpret_cast<const __half2*>(&w));
+    return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
 // ---------------------------------------------------------------------------------------------
-// The expert kernel. Grid: (N / (16 * RT * tiles_per_warp), items) with RT = WARPS / KS row tiles side
-// by side in a CTA; a warp walks `tiles_per_warp` consecutive 16-row tiles, and its cp.async ring keeps
-// streaming across the tile boundaries.
-//   NMAT = 2: gate/up + SwiGLU into hbuf.   NMAT = 1: down projection into the router positions.
-//   KS: warps that split K for one row tile (partials added in warp order through shared memory).
+// The streaming kernel.
+//   KS: warps that share one row tile, splitting K; the CTA works on RT = warps / KS tiles at a time.
+//   NBUF: staged passes (2: the next pass's rows are converted while this one is multiplied).
 // ---------------------------------------------------------------------------------------------
-//   MW: 1 = a warp streams all NMAT matrices of its rows; 2 (gate/up only) = gate and up of the same rows
-//       go to two different warps, which halves the registers and ring of a warp (three CTAs per SM instead
-//       of two) at the price of meeting in shared memory for the SwiGLU.
-//   CH: quantisation groups per ring stage (4 when K is a multiple of 256, else 2; Q8 always 2).
-//   MBG: scales and biases arrive MBG = 8 or 4 groups at a time (needs KS = 1 and a group count that is a multiple of MBG); 0: with every ring stage.
-template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH, int MBG>
-__global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN : (MW == 2 ? 3 : ZC_MIN_BLOCKS)) expert_kernel(Call c, uint32_t tiles_per_warp) {
-    using F = Fmt<BITS, CH>;
-    constexpr int STAGES = stages_for(NMAT / MW, CH);
-    constexpr int WM = NMAT / MW;                    // matrices per warp
-    constexpr int RT = WARPS / (KS * MW);
-    constexpr int STAGE = WM * F::MATRIX;
-    constexpr int META_AREA = F::meta_area(MBG, STAGES);
-    constexpr bool MB8 = MBG != 0;                   // metadata in blocks of MBG groups
-    constexpr int MBLOCK = MBG ? MBG : 8;
-    constexpr bool VIA_SMEM = KS > 1 || MW > 1;
-    constexpr int WORDS = F::ROWB / 16;              // 32-bit words per lane per row per group: 2 (Q4) / 4 (Q8)
+template <int BITS, bool SPLIT, bool FOLD, bool META_F16, int NMAT>
+__global__ void __launch_bounds__(MAX_THREADS, 1) stream_kernel(const Call c, const __grid_constant__ StreamMaps maps, const StreamPlan plan) {
+    constexpr int GPS = BITS == 4 ? 4 : 2;           // quantisation groups of one stage (128 code bytes of a row)
+    constexpr int TILE = NMAT == 2 ? 16 : 32;        // matrix rows of a warp's tile; a stage holds two 16-row fragments either way
+    constexpr int WORDS = BITS / 2;                  // 32-bit words per lane per row per group
     constexpr bool FOLDQ = FOLD && BITS == 4;
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    // gate/up follows the routing kernel and needs its lists at once. down follows gate/up, whose own wait has
-    // already seen the routing kernel complete: the item, the row lists and the first weight stages of down are
-    // set up while gate/up is still draining, and only the read of the SwiGLU rows waits for it.
-    if constexpr (NMAT == 2) { pdl_wait(); pdl_launch_dependents(); }
-    ItemInfo it;
-    if (!decode_item(c, blockIdx.y, it)) return;
-    const uint32_t K = NMAT == 2 ? c.H : c.F, G = K / 64, RS = K + ROW_PAD;
-    __half* xhi = reinterpret_cast<__half*>(smem_raw);
-    __half* xlo = xhi + (SPLIT ? NTOK * RS : 0);
-    float* sums = reinterpret_cast<float*>(xhi + (SPLIT ? 2 : 1) * NTOK * RS);       // [G][NTOK][2]
-    uint8_t* ring = reinterpret_cast<uint8_t*>(sums + G * NTOK * 2);                  // [WARPS][STAGES][STAGE]
-    uint8_t* meta_all = ring + WARPS * STAGES * STAGE;                                // [WARPS][WM][META_AREA]
-    float* red = reinterpret_cast<float*>(meta_all + WARPS * WM * META_AREA);      // [KS][NMAT][RT*16][NTOK] when VIA_SMEM
-    __shared__ int rows[NTOK];
-    __shared__ long long dest[NTOK];
+    constexpr int SW = GPS / 2;                      // words of a row's scales in one stage
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(16) uint64_t ring_bar[MAX_WARPS][STAGES];
+    __shared__ __align__(16) uint64_t rows_full[2], rows_done[2];      // per staged pass: every warp has converted its share / has finished its tiles
+    __shared__ int4 table[TABLE];                    // {expert (-1: shared), first position, rows, first row in hbuf}
+    __shared__ int slots[TABLE][NROW];               // gate/up: token of every row; down: its router slot (routed) or token (shared); -1: absent
+    __shared__ uint32_t warp_sums[MAX_WARPS];
+    __shared__ int perm_s[PERM_CACHE];
 
-    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, cq = lane % 4;
-    const uint32_t mw = warp % MW, ks = (warp / MW) % KS, rt = warp / (MW * KS);
-    const uint32_t first_tile = (blockIdx.x * RT + rt) * tiles_per_warp;
-    uint8_t* my_ring = ring + warp * STAGES * STAGE;
-    uint8_t* my_meta = meta_all + warp * WM * META_AREA;
-    const uint32_t nchunks = G / CH;                 // G is a multiple of CH
-    const uint32_t my_n = ks < nchunks ? (nchunks - ks + KS - 1) / KS : 0;
-    const uint32_t my_tiles = my_n ? tiles_per_warp : 0;
-    const bool q8s = c.q8_signed;
-    float* out_base = it.shared ? c.shared_out : c.expert_out;
-    LaneSource<BITS, CH> src[WM];
-#pragma unroll
-    for (int j = 0; j < WM; ++j) {
-        const uint32_t mi = mw * WM + j;             // 0 = gate (or down), 1 = up
-        src[j].init(it.record, NMAT == 1 ? c.down : (mi == 0 ? c.gate : c.up), lane, G);
+    const uint32_t W = plan.warps, KS = plan.ks, RT = plan.rt, NBUF = plan.nbuf, UB = plan.tiles_per_pass, pairs = plan.pairs;
+    const uint32_t tid = threadIdx.x, lane = tid % 32, g = lane / 4, cq = lane % 4;
+    const uint32_t warp = __shfl_sync(0xffffffffu, tid / 32, 0);       // warp-uniform for the compiler too
+    const uint32_t ks = warp & (KS - 1), rt = warp >> plan.ks_shift;
+    const uint32_t K = NMAT == 2 ? c.H : c.F, N = NMAT == 2 ? c.F : c.H, G = K / 64;
+    const uint32_t GPAD = pairs * 2 * GPS, RS = GPAD * 64 + ROW_PAD, GP = GPAD + 8;
+    const uint32_t buf_bytes = (SPLIT ? 2 : 1) * NROW * RS * 2 + NROW * GP * 4 + GPAD * NROW * 8;
+    uint8_t* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* rows_base = ring + W * STAGES * STAGE_BYTES;                             // [NBUF]: hi [NROW][RS], lo, sx [NROW][GP], offs [GPAD][NROW / 2][4]
+    float* red = reinterpret_cast<float*>(rows_base + NBUF * buf_bytes);              // [RT][KS - 1][2][32] float4
+    auto hi_of = [&](uint32_t buf) { return reinterpret_cast<__half*>(rows_base + buf * buf_bytes); };
+    auto sx_of = [&](uint32_t buf) { return reinterpret_cast<float*>(rows_base + buf * buf_bytes + (SPLIT ? 2 : 1) * NROW * RS * 2); };
+    const uint32_t ring_base = smem_u32(ring) + warp * (STAGES * STAGE_BYTES), bar_base = smem_u32(&ring_bar[0][0]) + warp * (STAGES * 8);
+    const uint32_t full_base = smem_u32(&rows_full[0]), done_base = smem_u32(&rows_done[0]);
+    if (tid < W * STAGES + 4) {
+        const uint32_t at = tid < W * STAGES ? smem_u32(&ring_bar[0][0]) + tid * 8 : tid < W * STAGES + 2 ? full_base + (tid - W * STAGES) * 8 : done_base + (tid - W * STAGES - 2) * 8;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(at), "r"(tid < W * STAGES ? 1u : W) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (GPAD != G) {                                 // k past the matrix: codes arrive as zeros and meet zeros
+        for (uint32_t buf = 0; buf < NBUF; ++buf) {
+            __half* xh = hi_of(buf);
+            float* sx = sx_of(buf);
+            float* offs = sx + NROW * GP;
+            for (uint32_t i = tid; i < (SPLIT ? 2 : 1) * NROW * (GPAD - G) * 64; i += blockDim.x)
+                xh[(i / ((GPAD - G) * 64)) * RS + G * 64 + i % ((GPAD - G) * 64)] = __ushort_as_half(0);
+            for (uint32_t i = tid; i < NROW * (GPAD - G); i += blockDim.x) {
+                const uint32_t n = i / (GPAD - G), grp = G + i % (GPAD - G);
+                sx[n * GP + grp] = 0.0f;
+                offs[grp * 2 * NROW + n] = offs[grp * 2 * NROW + NROW + n] = 0.0f;
+            }
+        }
     }
 
-    // An item with more than eight rows takes several passes; with gridDim.z > 1 they are spread over that many CTAs
-    // (a pass is independent of the others), so that one long item does not set the duration of a launch.
-    for (uint32_t pass = blockIdx.z; pass * NTOK < it.count; pass += gridDim.z) {
-        const uint32_t nvalid = min(uint32_t(NTOK), it.count - pass * NTOK);
-        uint32_t is_tile = 0, is_chunk = 0, is_slot = 0;        // producer position in the flattened (tile, chunk) sequence
-        uint32_t is_mblk = 0;                  // MB8: metadata blocks issued so far; the next one goes to buffer is_mblk & 1
-        const uint32_t ring_base = smem_u32(my_ring), meta_base = smem_u32(my_meta);
+    // gate/up follows the routing kernel and needs its lists at once. down follows gate/up, whose own wait has
+    // already seen the routing kernel complete: the passes, the row lists and the first weight stages of down are
+    // set up while gate/up is still draining, and only the read of the SwiGLU rows waits for it.
+    uint32_t limit = POLL_LIMIT, parity0 = 0, parity1 = 0, done_tiles = 0, fin = rt & (KS - 1);
+    if constexpr (NMAT == 2) { pdl_wait(); pdl_launch_dependents(); }
+
+    // ---- the passes: the shared expert's blocks of NROW tokens, then every listed expert's blocks of NROW rows ----
+    const uint32_t shared_passes = c.has_shared ? (c.T + NROW - 1) / NROW : 0;
+    // A thread owns `own` consecutive entries of the item list; the first stays in registers, others (more experts than
+    // threads) are read again when the table is filled.
+    const uint32_t own = plan.own;
+    auto entry_at = [&](uint32_t q) {
+        int4 e = make_int4(-1, 0, 0, 0);
+        if (tid * own + q < c.E) e = __ldcg(c.items + tid * own + q);                  // x = -1 past the list's end
+        if (e.x < 0 || (c.item_rows_max && uint32_t(e.z) > c.item_rows_max)) e.z = 0;  // those rows go to the tensor-core family
+        return e;
+    };
+    const uint32_t slots_total = c.T * c.K;
+    const bool perm_cached = slots_total <= PERM_CACHE;
+    int perm_mine[2] = {0, 0};
+    if (perm_cached) {
 #pragma unroll
-        for (int m = 0; m < WM; ++m) src[m].set_tile(first_tile * 16, G);
-        auto issue = [&]() {
-            if (is_tile < my_tiles) {
-                const uint32_t stage = ring_base + is_slot * STAGE, grp0 = (ks + is_chunk * KS) * CH;
-                const bool meta_now = MB8 && (is_chunk * CH) % MBLOCK == 0;
-                const uint32_t meta_buf = MB8 ? (is_mblk & 1) : is_slot;
+        for (int q = 0; q < 2; ++q) if (tid + q * blockDim.x < slots_total) perm_mine[q] = __ldcg(c.perm + tid + q * blockDim.x);
+    }
+    const int4 entry0 = entry_at(0);
+    uint32_t mine = (uint32_t(entry0.z) + NROW - 1) / NROW;
+    for (uint32_t q = 1; q < own; ++q) mine += (uint32_t(entry_at(q).z) + NROW - 1) / NROW;
+    if (perm_cached) {
 #pragma unroll
-                for (int m = 0; m < WM; ++m) issue_matrix<BITS, CH, MBG>(stage + m * F::MATRIX, meta_base + m * META_AREA, src[m], grp0, meta_buf, meta_now);
-                if (meta_now) ++is_mblk;
-                if (++is_chunk == my_n) {
-                    is_chunk = 0; ++is_tile;
+        for (int q = 0; q < 2; ++q) if (tid + q * blockDim.x < slots_total) perm_s[tid + q * blockDim.x] = perm_mine[q];
+        for (uint32_t i = tid + 2 * blockDim.x; i < slots_total; i += blockDim.x) perm_s[i] = __ldcg(c.perm + i);
+    }
+    uint32_t before = mine;
 #pragma unroll
-                    for (int m = 0; m < WM; ++m) src[m].set_tile((first_tile + is_tile) * 16, G);
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, before, off);
+        if (lane >= uint32_t(off)) before += v;
+    }
+    if (lane == 31) warp_sums[warp] = before;
+    __syncthreads();
+    uint32_t total_passes = shared_passes;
+    before += shared_passes - mine;
+    {
+        const uint32_t v = lane < W ? warp_sums[lane] : 0;
+        total_passes += __reduce_add_sync(0xffffffffu, v);
+        before += __reduce_add_sync(0xffffffffu, lane < warp ? v : 0);
+    }
+    // Tiles of all passes end to end; this CTA takes [t_first, t_last), its group rt every RT-th of them.
+    const uint32_t tiles = total_passes * UB, each = quick_div(tiles, gridDim.x, plan.inv_grid), extra = tiles - each * gridDim.x;
+    const uint32_t t_first = blockIdx.x * each + min(blockIdx.x, extra), t_last = t_first + each + (blockIdx.x < extra ? 1u : 0u);
+    if (t_first == t_last) { if (NMAT == 1) pdl_wait(); return; }
+
+    const uint32_t pi = ((g & 1) << 2) | (g & 2) | (g >> 2);                          // tile row of MMA row g
+    const uint32_t lane_off = BITS == 4 ? pi * 128 + ((((cq >> 1) ^ pi) << 4) | ((cq & 1) << 3)) : pi * 128 + ((cq ^ pi) << 4);
+    const uint8_t* code_at[GPS];                     // the lane's codes of row g of the first fragment, per group of a stage
+#pragma unroll
+    for (int j = 0; j < GPS; ++j) code_at[j] = ring + warp * (STAGES * STAGE_BYTES) + (BITS == 4 ? (lane_off ^ uint32_t(j << 5)) : (lane_off ^ uint32_t(j << 6)));
+    const bool q8s = c.q8_signed;
+    bool waited = NMAT == 2;
+    const uint32_t meta_at = NMAT == 2 ? uint32_t(c.gate.scales) : uint32_t(c.down.scales);
+    const uint32_t meta_frag = NMAT == 2 ? uint32_t(c.up.scales - c.gate.scales) : 16 * G * 2;       // second fragment: the same rows of up, or the next 16 rows of down
+    const uint32_t bias_at = N * G * 2 + cq * (BITS == 4 ? 4 : 2), lane_scale = pi * (G * 2), step_bytes = KS * (2 * GPS) * 2;
+    const bool whole_pairs = G % (2 * GPS) == 0;
+    const uint32_t stages = (G + GPS - 1) / GPS;     // of a row's K; odd: the last pair has one
+    auto wait_bar = [&](uint32_t bar, uint32_t ph) {       // bounded; a second full wait lets a late copy land before its buffer is used again
+        if (ring_wait(bar, ph, limit)) return;
+        atomicOr(c.status, ZC_STATUS_TIMEOUT);
+        ring_wait(bar, ph, limit);
+        limit = 16;
+    };
+
+    const uint32_t p_first = quick_div(t_first, UB, plan.inv_tiles), p_last = quick_div(t_last - 1, UB, plan.inv_tiles);
+    for (uint32_t pw = p_first; pw <= p_last; pw += TABLE) {
+        const uint32_t np = min(p_last - pw + 1, uint32_t(TABLE));                    // passes of this window
+        const uint32_t ta = max(t_first, pw * UB), tb = min(t_last, (pw + np) * UB);  // its tiles
+        if (pw != p_first) __syncthreads();                                           // the previous window's entries have been read
+        if (tid < np && pw + tid < shared_passes) {
+            const uint32_t p0 = (pw + tid) * NROW;
+            table[tid] = make_int4(-1, int(p0), int(min(uint32_t(NROW), c.T - p0)), int(c.T * c.K + p0));
+        }
+        {
+            uint32_t first = before;
+            for (uint32_t q = 0; q < own; ++q) {
+                const int4 e = q == 0 ? entry0 : entry_at(q);
+                const uint32_t n = (uint32_t(e.z) + NROW - 1) / NROW;
+                for (uint32_t p = max(first, pw); p < min(first + n, pw + np); ++p) {
+                    const uint32_t r0 = (p - first) * NROW, pos = uint32_t(e.y) + r0;
+                    table[p - pw] = make_int4(e.x - int(c.first_expert), int(pos), int(min(uint32_t(NROW), uint32_t(e.z) - r0)), int(pos));
                 }
+                first += n;
             }
-            cp_async_commit();
-            is_slot = is_slot + 1 == STAGES ? 0 : is_slot + 1;
-        };
-        __syncthreads();                       // everything of the previous pass has been consumed
-#pragma unroll
-        for (int i = 0; i < STAGES - 1; ++i) issue();    // weights do not depend on the rows: start them first
-        if (threadIdx.x < NTOK) {
-            const uint32_t i = pass * NTOK + threadIdx.x;
-            if (i < it.count) {
-                if (NMAT == 2) rows[threadIdx.x] = it.shared ? int(it.pos0 + i) : c.perm[it.pos0 + i] / int(c.K);
-                else rows[threadIdx.x] = int(it.hrow0 + i);
-                const uint32_t slot = it.shared ? it.pos0 + i : uint32_t(c.perm[it.pos0 + i]);
-                dest[threadIdx.x] = NMAT == 2 ? (long long)(it.hrow0 + i) * c.F : (long long)slot * c.H;
-            } else { rows[threadIdx.x] = -1; dest[threadIdx.x] = -1; }
         }
         __syncthreads();
-        if constexpr (NMAT == 1) { pdl_wait(); pdl_launch_dependents(); }
-        stage_rows<BITS == 4, SPLIT, FOLDQ>(NMAT == 2 ? c.x : static_cast<const void*>(c.hbuf), NMAT == 2 ? c.act_dtype == ZC_F32 : true,
-                                            rows, nvalid, K, c.ref && BITS == 4, xhi, xlo, sums, c.status);
-        __syncthreads();
 
-        // The lane holds rows g, g+8 of its tile for tokens 2cq, 2cq+1.
-        auto finish = [&](uint32_t row, uint32_t n, float a0, float a1) {
-            const long long d = dest[n];
-            if (d < 0) return;
-            if constexpr (FOLDQ) { a0 *= 0.0625f; a1 *= 0.0625f; }          // the rows were staged x 16
-            if constexpr (NMAT == 2) {
-                float h;
-                if (c.ref) {   // qwen.metal:71-81
-                    const float gate = bf_round(a0), up = bf_round(a1);
-                    h = bf_round(bf_round(gate * sigmoid_bf(gate)) * up);
-                } else {
-                    h = (a0 * sigmoid_f(a0)) * a1;
-                }
-                c.hbuf[d + row] = h;
-            } else {
-                out_base[d + row] = c.ref ? bf_round(a0) : a0;
-            }
+        // ---- the sequence of this warp: pairs of stages (2 GPS groups) of its tiles. While a pair is multiplied, each of its
+        // two ring slots is refilled with the next pair's stage as soon as it has been read, and the stage's scales and the
+        // pair's biases are fetched for the next pair into the registers they leave ----
+        struct Cursor { uint32_t t, blk, ps; };      // tile of the window's sequence, its place in its pass, its pass in the table
+        auto next_tile = [&](Cursor& k) { k.t += RT; k.blk += RT; while (k.blk >= UB) { k.blk -= UB; ++k.ps; } };
+        Cursor now{ta, pw == p_first ? t_first - p_first * UB : 0, 0};
+        now.t += rt; now.blk += rt;
+        while (now.blk >= UB) { now.blk -= UB; ++now.ps; }
+        Cursor ahead = now;                          // the tile of the next pair, and the pair
+        uint32_t ahead_pair = ks;
+        int ahead_e = 0;
+        const CUtensorMap* ahead_map = &maps.routed;
+        const uint8_t* mp[2][2];                     // the lane's scale pointers: [fragment][row g / g+8] of the next pair
+        auto enter_tile = [&]() {                    // ahead.t < tb
+            const int e = __shfl_sync(0xffffffffu, table[ahead.ps].x, 0);
+            ahead_e = max(e, 0);
+            ahead_map = e < 0 ? &maps.shared : &maps.routed;
+            const uint8_t* rec = (e < 0 ? c.shared_record : c.records + size_t(e) * c.record_stride) + (meta_at + ahead.blk * TILE * (G * 2) + ks * (2 * GPS * 2)) + lane_scale;
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) mp[m][r] = rec + (m * meta_frag + r * G * 16);
         };
-
-        uint32_t slot = 0, mblk = 0;           // mblk: metadata blocks the consumer has begun (MB8)
-        for (uint32_t tile = 0; tile < tiles_per_warp; ++tile) {
-            float acc[WM][4];
+        uint32_t sc[2][2][2][SW];                    // [stage of the pair][fragment][row g / g+8]: the scales of the stage's groups, two per word
+        uint32_t bi[2][2];                           // the biases this lane supplies to the pair's bias product
+        auto issue = [&](int half) {
+            if (lane == 0 && ahead_pair * 2 + half < stages) ring_load(ring_base + half * STAGE_BYTES, ahead_map, bar_base + half * 8, int((ahead_pair * 2 + half) * 128), int(ahead.blk * TILE), ahead_e);
+        };
+        auto fetch_scales = [&](int half) {
 #pragma unroll
-            for (int m = 0; m < WM; ++m) { acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.0f; }
-            for (uint32_t i = 0; i < my_n; ++i) {
-                cp_async_wait<STAGES - 2>();
-                __syncwarp();
-                const uint8_t* stage = my_ring + slot * STAGE;
-                // this chunk's scale and bias halves: at its place in the current 8-group block (MB8), or in the buffer of its slot
-                if (MB8 && (i * CH) % MBLOCK == 0) ++mblk;
-                constexpr uint32_t PAIR = MB8 ? uint32_t(MBLOCK * 2) : uint32_t(CH * 2);          // bytes of one (row, kind) entry
-                const uint8_t* mbase = MB8 ? my_meta + ((mblk - 1) & 1) * (32 * PAIR) + ((i * CH) % MBLOCK) * 2 : my_meta + slot * (32 * CH * 2);
-                slot = slot + 1 == STAGES ? 0 : slot + 1;
-                issue();          // refills the slot consumed by the previous iteration while this chunk is multiplied
-                const uint32_t grp0 = (ks + i * KS) * CH;
-                uint32_t mraw[WM][2][CH];                        // per row: CH scale halves then CH bias halves, two per word
+            for (int m = 0; m < 2; ++m)
 #pragma unroll
-                for (int m = 0; m < WM; ++m) {
+                for (int r = 0; r < 2; ++r) {
+                    const uint8_t* p = mp[m][r] + half * (GPS * 2);
+                    if (whole_pairs) {
+                        if constexpr (GPS == 4) {
+                            const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+                            sc[half][m][r][0] = v.x; sc[half][m][r][SW - 1] = v.y;
+                        } else sc[half][m][r][0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+                    } else {                         // rows of an even number of groups: words are 4-byte aligned, those past the row are zero
 #pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const uint8_t* mp = mbase + m * META_AREA + (g + 8 * r) * 2 * PAIR;
-                        if constexpr (CH == 4) {
-                            const uint2 sc = *reinterpret_cast<const uint2*>(mp), bi = *reinterpret_cast<const uint2*>(mp + PAIR);
-                            mraw[m][r][0] = sc.x; mraw[m][r][1] = sc.y; mraw[m][r][2] = bi.x; mraw[m][r][3] = bi.y;
-                        } else if constexpr (MB8) {
-                            mraw[m][r][0] = *reinterpret_cast<const uint32_t*>(mp); mraw[m][r][1] = *reinterpret_cast<const uint32_t*>(mp + PAIR);
-                        } else {
-                            const uint2 v = *reinterpret_cast<const uint2*>(mp);
-                            mraw[m][r][0] = v.x; mraw[m][r][1] = v.y;
-                        }
+                        for (int w = 0; w < SW; ++w)
+                            sc[half][m][r][w] = (ahead_pair * 2 + half) * GPS + 2 * w < G ? __ldg(reinterpret_cast<const uint32_t*>(p) + w) : 0u;
                     }
                 }
-                // scale / bias of row r (0: g, 1: g+8) for group j of the chunk, converted where it is used
-                auto meta_of = [&](int m, int r, int j, bool bias) {
-                    const uint32_t word = mraw[m][r][(bias ? CH / 2 : 0) + j / 2];
-                    const uint16_t bits = (j & 1) ? uint16_t(word >> 16) : uint16_t(word & 0xffffu);
-                    return META_F16 ? __half2float(__ushort_as_half(bits)) : bf_to_float(bits);
-                };
+        };
+        auto fetch_biases = [&]() {
+            const bool on = whole_pairs || ahead_pair * (2 * GPS) + (BITS == 4 ? 2 * cq : cq) < G;
 #pragma unroll
-                for (int j = 0; j < CH; ++j) {
-                    const uint32_t grp = grp0 + j;
-                    uint4 bh[2], bl[2];
-                    bh[0] = bh[1] = bl[0] = bl[1] = make_uint4(0, 0, 0, 0);
-                    if (g < nvalid) {             // lanes of absent token rows skip the reads (their MMA columns are never stored)
-                        const __half* bp = xhi + g * RS + grp * 64 + cq * 16;
-                        bh[0] = *reinterpret_cast<const uint4*>(bp);
-                        bh[1] = *reinterpret_cast<const uint4*>(bp + 8);
-                        if constexpr (SPLIT) {
-                            const __half* lp = xlo + g * RS + grp * 64 + cq * 16;
-                            bl[0] = *reinterpret_cast<const uint4*>(lp);
-                            bl[1] = *reinterpret_cast<const uint4*>(lp + 8);
-                        }
-                    }
-                    const float4 sm = *reinterpret_cast<const float4*>(sums + (grp * NTOK + 2 * cq) * 2);   // (Sx, P) of tokens 2cq, 2cq+1
+            for (int m = 0; m < 2; ++m)
 #pragma unroll
-                    for (int m = 0; m < WM; ++m) {
-                        const uint8_t* ms = stage + m * F::MATRIX;
-                        uint32_t w0[WORDS], w1[WORDS];
-                        const uint32_t blk = ((uint32_t(j) ^ F::swizzle(g)) * F::ROWB);           // swizzle(g + 8) == swizzle(g)
-                        if constexpr (BITS == 4) {
-                            const uint2 a = *reinterpret_cast<const uint2*>(ms + g * F::LINE + blk + cq * 8);
-                            const uint2 b = *reinterpret_cast<const uint2*>(ms + (g + 8) * F::LINE + blk + cq * 8);
-                            w0[0] = a.x; w0[1] = a.y; w1[0] = b.x; w1[1] = b.y;
-                        } else {
-                            const uint4 a = *reinterpret_cast<const uint4*>(ms + g * F::LINE + blk + cq * 16);
-                            const uint4 b = *reinterpret_cast<const uint4*>(ms + (g + 8) * F::LINE + blk + cq * 16);
-                            w0[0] = a.x; w0[1] = a.y; w0[2] = a.z; w0[3] = a.w; w1[0] = b.x; w1[1] = b.y; w1[2] = b.z; w1[3] = b.w;
-                        }
-                        float d[4];
-                        group_mma<BITS, SPLIT, FOLDQ>(d, sm.y, sm.w, w0, w1, bh, bl, q8s);    // starts from P: removes the folded offset
-                        const float s0 = meta_of(m, 0, j, false), s1 = meta_of(m, 1, j, false), b0 = meta_of(m, 0, j, true), b1 = meta_of(m, 1, j, true);
-                        acc[m][0] = __fmaf_rn(s0, d[0], acc[m][0]); acc[m][0] = __fmaf_rn(b0, sm.x, acc[m][0]);
-                        acc[m][1] = __fmaf_rn(s0, d[1], acc[m][1]); acc[m][1] = __fmaf_rn(b0, sm.z, acc[m][1]);
-                        acc[m][2] = __fmaf_rn(s1, d[2], acc[m][2]); acc[m][2] = __fmaf_rn(b1, sm.x, acc[m][2]);
-                        acc[m][3] = __fmaf_rn(s1, d[3], acc[m][3]); acc[m][3] = __fmaf_rn(b1, sm.z, acc[m][3]);
-                    }
+                for (int r = 0; r < 2; ++r) {
+                    if constexpr (BITS == 4) bi[m][r] = on ? __ldg(reinterpret_cast<const uint32_t*>(mp[m][r] + bias_at)) : 0u;
+                    else bi[m][r] = on ? uint32_t(__ldg(reinterpret_cast<const uint16_t*>(mp[m][r] + bias_at))) : 0u;
                 }
-                __syncwarp();
+        };
+        auto step = [&]() {                          // `ahead` to the pair after it
+            ahead_pair += KS;
+            if (ahead_pair < pairs) {
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) mp[m][r] += step_bytes;
+                return;
             }
-            const uint32_t cta_row0 = blockIdx.x * RT * tiles_per_warp * 16;
-            if constexpr (!VIA_SMEM) {
-                const uint32_t row0 = (first_tile + tile) * 16;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) finish(row0 + g + 8 * (i >> 1), 2 * cq + (i & 1), acc[0][i], acc[WM - 1][i]);
-            } else {
-                // partials: [ks][matrix][row tile in CTA][row][token]
-#pragma unroll
-                for (int m = 0; m < WM; ++m) {
-                    float* mine = red + ((ks * NMAT + mw * WM + m) * RT * 16 + rt * 16) * NTOK;
-                    *reinterpret_cast<float2*>(mine + g * NTOK + 2 * cq) = make_float2(acc[m][0], acc[m][1]);
-                    *reinterpret_cast<float2*>(mine + (g + 8) * NTOK + 2 * cq) = make_float2(acc[m][2], acc[m][3]);
+            ahead_pair = ks;
+            next_tile(ahead);
+            if (ahead.t < tb) enter_tile();
+        };
+        // rows of this window's passes
+        for (uint32_t i = tid; i < np * NROW; i += blockDim.x) {
+            const int4 d = table[i / NROW];
+            const uint32_t n = i % NROW;
+            int v = -1;
+            if (int(n) < d.z) {
+                if (d.x < 0) v = d.y + int(n);
+                else {
+                    v = perm_cached ? perm_s[d.y + n] : __ldcg(c.perm + d.y + n);
+                    if (NMAT == 2) v = int(uint32_t(v) / c.K);
                 }
-                __syncthreads();
-                for (uint32_t o = threadIdx.x; o < RT * 16 * NTOK; o += EXPERT_THREADS) {
-                    const uint32_t r = o / NTOK, n = o % NTOK;
-                    float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < KS; ++k) {
-                        a0 += red[((k * NMAT + 0) * RT * 16 + r) * NTOK + n];
-                        if constexpr (NMAT == 2) a1 += red[((k * NMAT + 1) * RT * 16 + r) * NTOK + n];
-                    }
-                    // row tile r/16 of this CTA walks tiles (blockIdx.x*RT + r/16) * tiles_per_warp + tile
-                    finish(cta_row0 + ((r / 16) * tiles_per_warp + tile) * 16 + r % 16, n, a0, a1);
-                }
-                __syncthreads();
             }
+            slots[i / NROW][n] = v;
         }
-        cp_async_wait<0>();
+        __syncthreads();
+        if (!waited) { pdl_wait(); pdl_launch_dependents(); waited = true; }
+
+        // This warp's share of the rows of pass q (counted from p_first), once the pass that used the buffer before is done.
+        auto stage_share = [&](uint32_t ps) {
+            const uint32_t q = pw + ps - p_first, buf = q & (NBUF - 1), use = NBUF == 2 ? q >> 1 : q;
+            if (use) wait_bar(done_base + buf * 8, (use - 1) & 1);
+            const int4 d = table[ps];
+            __half* hi = hi_of(buf);
+            float* sx = sx_of(buf);
+            stage_rows<BITS == 4, SPLIT, FOLDQ>(NMAT == 2 ? c.x : static_cast<const void*>(c.hbuf), NMAT == 2 ? c.act_dtype == ZC_F32 : true,
+                [&](uint32_t n) { return NMAT == 2 ? size_t(slots[ps][n]) : size_t(d.w) + n; },
+                uint32_t(d.z), K, RS, GP, c.ref && BITS == 4, hi, hi + NROW * RS, sx, sx + NROW * GP, c.status, warp, W);
+            __syncwarp();
+            if (lane == 0) bar_arrive(full_base + buf * 8);
+        };
+        // The rows of the first pass are requested before the first weights, which would otherwise stand in front of them in
+        // the memory system (128 KB per SM at once); those of the second pass (two blocks) behind them.
+        const bool any = ahead.t < tb;
+        if (any) { enter_tile(); issue(0); }
+#pragma unroll 1
+        for (uint32_t ps = 0; ps < min(np, NBUF); ++ps) stage_share(ps);
+        if (any) {
+            issue(1);
+            fetch_scales(0);
+            fetch_scales(1);
+            fetch_biases();
+            step();
+        }
+        for (uint32_t ps = 0; ps < np; ++ps) {
+            const uint32_t q = pw + ps - p_first, buf = q & (NBUF - 1), use = NBUF == 2 ? q >> 1 : q;
+            bool next_staged = ps + 1 == np || (NBUF == 2 && ps == 0);   // the window's second pass already is
+            wait_bar(full_base + buf * 8, use & 1);
+            const uint32_t nvalid = uint32_t(__shfl_sync(0xffffffffu, table[ps].z, 0));
+            const __half* xhi = hi_of(buf);
+            const __half* xlo = xhi + NROW * RS;
+            const float* sx = sx_of(buf);
+            const float* offs = sx + NROW * GP;
+            const uint32_t row_at = g < nvalid ? g : 0;                  // the lane's token row in the staged block; lanes without one read row 0 (their MMA columns are never stored)
+            bool more = now.ps == ps && now.t < tb, left = false;
+            do {
+                if (more) {
+                    float acc[2][4] = {};
+                    for (uint32_t pair = ks; pair < pairs; pair += KS) {
+                        const float4* op = reinterpret_cast<const float4*>(offs) + pair * (2 * GPS) * (NROW / 2) + cq;
+                        const __half* xb = xhi + row_at * RS + pair * (2 * GPS * 64) + cq * 16;
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+                            if (half == 0 || pair * 2 + 1 < stages) {
+                                wait_bar(bar_base + half * 8, half ? parity1 : parity0);
+                                if (half) parity1 ^= 1; else parity0 ^= 1;
+#pragma unroll
+                                for (int j = 0; j < GPS; ++j) {
+                                    const __half* x = xb + (half * GPS + j) * 64;
+                                    const uint4 bh[2] = {*reinterpret_cast<const uint4*>(x), *reinterpret_cast<const uint4*>(x + 8)};
+                                    uint4 bl[2] = {};
+                                    if constexpr (SPLIT) {
+                                        bl[0] = *reinterpret_cast<const uint4*>(x + NROW * RS);
+                                        bl[1] = *reinterpret_cast<const uint4*>(x + NROW * RS + 8);
+                                    }
+                                    const float4 off = FOLDQ ? op[(half * GPS + j) * (NROW / 2)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                                    uint32_t w[2][2][WORDS];
+#pragma unroll
+                                    for (int m = 0; m < 2; ++m)
+#pragma unroll
+                                        for (int r = 0; r < 2; ++r) {
+                                            const uint8_t* at = code_at[j] + half * STAGE_BYTES + m * 2048 + r * 1024;
+                                            if constexpr (BITS == 4) {
+                                                const uint2 v = *reinterpret_cast<const uint2*>(at);
+                                                w[m][r][0] = v.x; w[m][r][1] = v.y;
+                                            } else {
+                                                const uint4 v = *reinterpret_cast<const uint4*>(at);
+                                                w[m][r][0] = v.x; w[m][r][1] = v.y; w[m][r][WORDS - 2] = v.z; w[m][r][WORDS - 1] = v.w;
+                                            }
+                                        }
+                                    float d[2][4];
+                                    group_mma<BITS, SPLIT, FOLDQ>(d, off, w, bh, bl, q8s);
+#pragma unroll
+                                    for (int m = 0; m < 2; ++m) {
+                                        const float2 p0 = meta_pair<META_F16>(sc[half][m][0][j / 2]), p1 = meta_pair<META_F16>(sc[half][m][1][j / 2]);
+                                        const float s0 = j % 2 ? p0.y : p0.x, s1 = j % 2 ? p1.y : p1.x;
+                                        acc[m][0] = __fmaf_rn(s0, d[m][0], acc[m][0]); acc[m][1] = __fmaf_rn(s0, d[m][1], acc[m][1]);
+                                        acc[m][2] = __fmaf_rn(s1, d[m][2], acc[m][2]); acc[m][3] = __fmaf_rn(s1, d[m][3], acc[m][3]);
+                                    }
+                                }
+                            }
+                            if (half == 1) {         // the bias product of the pair's groups
+                                const float* sp = sx + row_at * GP + pair * (2 * GPS);
+                                if constexpr (BITS == 4) {           // k slots cq and cq + 4 of the MMA are groups 2 cq and 2 cq + 1
+                                    const float2 v = *reinterpret_cast<const float2*>(sp + 2 * cq);
+                                    const float h0 = __uint_as_float(__float_as_uint(v.x) & 0xffffe000u), h1 = __uint_as_float(__float_as_uint(v.y) & 0xffffe000u);
+#pragma unroll
+                                    for (int m = 0; m < 2; ++m) {
+                                        const float2 b0 = meta_pair<META_F16>(bi[m][0]), b1 = meta_pair<META_F16>(bi[m][1]);
+                                        mma_tf32_1688(acc[m], b0.x, b1.x, b0.y, b1.y, h0, h1);
+                                        mma_tf32_1688(acc[m], b0.x, b1.x, b0.y, b1.y, v.x - h0, v.y - h1);
+                                    }
+                                } else {                             // k slot cq is group cq
+                                    const float v = sp[cq], h = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+#pragma unroll
+                                    for (int m = 0; m < 2; ++m) {
+                                        const float b0 = meta_pair<META_F16>(bi[m][0]).x, b1 = meta_pair<META_F16>(bi[m][1]).x;
+                                        mma_tf32_1684(acc[m], b0, b1, h);
+                                        mma_tf32_1684(acc[m], b0, b1, v - h);
+                                    }
+                                }
+                            }
+                            __syncwarp();            // every lane has read the stage: refill it
+                            if (ahead.t < tb) {
+                                issue(half);
+                                fetch_scales(half);
+                                if (half == 1) { fetch_biases(); step(); }
+                            }
+                        }
+                    }
+                    // ---- the KS partial sums of the tile, added in warp order by one of its warps ----
+                    bool finisher = true;
+                    if (KS > 1) {
+                        const uint32_t threads = KS * 32;
+                        finisher = ks == fin;
+                        // Barrier 1 + 2 rt: the partials are written. Barrier 2 + 2 rt: those of the tile before have been read. All
+                        // KS warps pass the second one before any of them arrives at the first again.
+                        if (done_tiles) group_sync(2 + 2 * rt, threads);
+                        float4* area = reinterpret_cast<float4*>(red) + size_t(rt) * (KS - 1) * 2 * 32 + lane;
+                        if (!finisher) {
+                            float4* to = area + size_t(ks < fin ? ks : ks - 1) * 2 * 32;
+#pragma unroll
+                            for (int m = 0; m < 2; ++m) to[m * 32] = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+                            group_arrive(1 + 2 * rt, threads);
+                        } else {
+                            group_sync(1 + 2 * rt, threads);
+                            float sum[2][4] = {};
+                            for (uint32_t k = 0; k < KS; ++k) {
+                                const float4* from = area + size_t(k < fin ? k : k - 1) * 2 * 32;
+#pragma unroll
+                                for (int m = 0; m < 2; ++m) {
+                                    const float4 v = k == fin ? make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]) : from[m * 32];
+                                    sum[m][0] += v.x; sum[m][1] += v.y; sum[m][2] += v.z; sum[m][3] += v.w;
+                                }
+                            }
+#pragma unroll
+                            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) acc[m][i] = sum[m][i];
+                        }
+                        fin = fin + 1 == KS ? 0 : fin + 1;
+                        ++done_tiles;
+                    }
+                    if (finisher) {                  // lane: rows pi, pi + 8 of the tile, tokens 2 cq, 2 cq + 1
+                        const uint32_t row0 = now.blk * TILE + pi;
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const uint32_t n = 2 * cq + i;
+                            if (n >= nvalid) continue;
+                            float a[2][2];
+#pragma unroll
+                            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                                for (int r = 0; r < 2; ++r) a[m][r] = FOLDQ ? acc[m][2 * r + i] * 0.0625f : acc[m][2 * r + i];       // the rows were staged x 16
+                            if constexpr (NMAT == 2) {
+                                float* to = c.hbuf + size_t(uint32_t(table[ps].w) + n) * c.F + row0;
+#pragma unroll
+                                for (int r = 0; r < 2; ++r) {
+                                    float h;
+                                    if (c.ref) {   // qwen.metal:71-81
+                                        const float gate = bf_round(a[0][r]), up = bf_round(a[1][r]);
+                                        h = bf_round(bf_round(gate * sigmoid_bf(gate)) * up);
+                                    } else {
+                                        h = (a[0][r] * sigmoid_f(a[0][r])) * a[1][r];
+                                    }
+                                    to[8 * r] = h;
+                                }
+                            } else {
+                                float* to = (table[ps].x < 0 ? c.shared_out : c.expert_out) + size_t(uint32_t(slots[ps][n])) * c.H + row0;
+#pragma unroll
+                                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                                    for (int r = 0; r < 2; ++r) to[16 * m + 8 * r] = c.ref ? bf_round(a[m][r]) : a[m][r];
+                            }
+                        }
+                    }
+                    next_tile(now);
+                    more = now.ps == ps && now.t < tb;
+                }
+                // The next pass's rows: after this warp's first tile of the pass (by then the others have left the pass before
+                // it, whose block they go to), with one block only when every warp is done with this pass.
+                if (!more && NBUF == 1) { left = true; __syncwarp(); if (lane == 0) bar_arrive(done_base + buf * 8); }
+                if (!next_staged && (NBUF == 2 || !more)) { next_staged = true; stage_share(ps + 1); }
+            } while (more);
+            if (!left) { __syncwarp(); if (lane == 0) bar_arrive(done_base + buf * 8); }
+        }
     }
 }
 
-template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH, int MBG>
-int launch_expert_mb(zc_moe* m, const Call& c, uint32_t items, uint32_t tiles_per_warp, cudaStream_t s) {
-    constexpr int RT = WARPS / (KS * MW);
-    constexpr int STAGES = stages_for(NMAT / MW, CH);
-    const uint32_t K = NMAT == 2 ? c.H : c.F, N = NMAT == 2 ? c.F : c.H, G = K / 64;
-    const size_t smem = size_t(SPLIT ? 2 : 1) * NTOK * (K + ROW_PAD) * 2 + size_t(G) * NTOK * 2 * 4 +
-                        size_t(WARPS) * (NMAT / MW) * (STAGES * Fmt<BITS, CH>::MATRIX + Fmt<BITS, CH>::meta_area(MBG, STAGES)) + ((KS > 1 || MW > 1) ? size_t(KS) * NMAT * RT * 16 * NTOK * 4 : 0);
-    if (smem > 220 * 1024) return fail(m, ZC_EINVAL, "expert kernel: shape needs too much shared memory");
-    while (tiles_per_warp > 1 && N % (16 * RT * tiles_per_warp)) --tiles_per_warp;
-    if (N % (16 * RT * tiles_per_warp)) return fail(m, ZC_EINVAL, "expert kernel: rows not a multiple of the CTA tile");
-    // Items that can have more than eight rows (two or more rows per expert on average, or the few-row side of a long
-    // batch with its limit above eight): their passes run as separate CTAs.
-    const uint32_t pass_ctas = (KS == 1 && (c.item_rows_max > NTOK || uint64_t(c.T) * c.K >= 2ull * c.local_experts)) ? 2u : 1u;
-    auto kernel = expert_kernel<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, MBG>;
+// Shared memory of a launch.
+size_t stream_smem(const StreamPlan& p, bool split, uint32_t K, uint32_t bits) {
+    const uint32_t gpad = p.pairs * (bits == 4 ? 8 : 4);
+    return 1024 + size_t(p.warps) * STAGES * STAGE_BYTES + size_t(p.warps / p.ks) * (p.ks - 1) * 2 * 32 * 16 +
+           p.nbuf * (size_t(split ? 2 : 1) * NROW * (gpad * 64 + ROW_PAD) * 2 + size_t(NROW) * (gpad + 8) * 4 + size_t(gpad) * NROW * 8);
+}
+constexpr size_t STREAM_SMEM_MAX = 221 * 1024;      // 227 KB less the static tables
+
+template <int BITS, bool SPLIT, bool FOLD, bool META_F16, int NMAT>
+int launch_stream(zc_moe* m, const Call& c, const StreamPlan& p, cudaStream_t s) {
+    const size_t smem = stream_smem(p, SPLIT, NMAT == 2 ? c.H : c.F, BITS);
+    auto kernel = stream_kernel<BITS, SPLIT, FOLD, META_F16, NMAT>;
     static SmemOptIn configured;        // one per instantiation of this function template
     if (opt_in_smem(kernel, configured, m->device, smem) != cudaSuccess) return check_launch(m, "expert kernel attribute");
+    const LayerMem& L = m->layers[c.layer];
+    const StreamMaps maps{NMAT == 2 ? L.map_gate_up.m : L.map_down.m, NMAT == 2 ? L.map_shared_gate_up.m : L.map_shared_down.m};
     Timed t(m, s, NMAT == 2 ? KERNEL_GATE_UP : KERNEL_DOWN);
-    const cudaError_t e = launch_chained(m, NMAT == 2 ? KERNEL_GATE_UP : KERNEL_DOWN, kernel, dim3(N / (16 * RT * tiles_per_warp), items, pass_ctas), dim3(EXPERT_THREADS), smem, s, nullptr, 0, c, tiles_per_warp);
+    const cudaError_t e = launch_chained(m, NMAT == 2 ? KERNEL_GATE_UP : KERNEL_DOWN, kernel, dim3(sm_count(m)), dim3(p.warps * 32), smem, s, nullptr, 0, c, maps, p);
     if (e != cudaSuccess) return fail(m, ZC_EEXEC, std::string("expert kernel launch: ") + cudaGetErrorString(e));
     return check_launch(m, NMAT == 2 ? "gate_up" : "down");
 }
 
-// Metadata in 8-group blocks: possible where a warp walks K in order (KS = 1) and every block of a row's metadata is
-// 16-byte aligned; used for gate/up with long rows (hidden 4096: 423 -> 368 us at 512 experts x 5 rows). With short rows
-// the extra kilobyte per warp pushes two CTAs per SM over a shared-memory carve-out step, which costs the L1 that serves
-// the small copies (97 -> 104 us at hidden 2048), and down's short K does not gain (56 -> 58 us): those keep one block per
-// ring stage. Option meta_blocks: 0 never, 1 by this rule, 2 wherever possible, 3 four-group blocks for gate/up.
-template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH>
-int launch_expert_ch(zc_moe* m, const Call& c, uint32_t items, uint32_t tiles_per_warp, cudaStream_t s) {
-    if constexpr (KS == 1) {
-        const uint32_t K = NMAT == 2 ? c.H : c.F, G = K / 64;
-        const bool long_rows = NMAT == 2 && K >= 4096;
-        if (G % 8 == 0 && (m->meta_blocks == 2 || (m->meta_blocks == 1 && long_rows)))
-            return launch_expert_mb<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, 8>(m, c, items, tiles_per_warp, s);
-        if constexpr (CH == 2 && NMAT == 2) {       // 4-group blocks (8-byte copies every second stage; stays inside the carve-out): 99.7 against 98.1 us at hidden 2048, so only on request
-            if (G % 4 == 0 && m->meta_blocks == 3)
-                return launch_expert_mb<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, 4>(m, c, items, tiles_per_warp, s);
-        }
-    }
-    return launch_expert_mb<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, 0>(m, c, items, tiles_per_warp, s);
+template <int BITS, bool FOLD, bool META_F16, int NMAT>
+int dispatch_split(zc_moe* m, const Call& c, const StreamPlan& p, bool split, cudaStream_t s) {
+    return split ? launch_stream<BITS, true, FOLD, META_F16, NMAT>(m, c, p, s) : launch_stream<BITS, false, FOLD, META_F16, NMAT>(m, c, p, s);
 }
-
-// Two groups per ring stage for gate/up: four groups per stage (a full 128-byte line per Q4 row) leave room for
-// only two stages next to the staged rows and measured 13 % slower at hidden 2048.
-template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW>
-int launch_expert(zc_moe* m, const Call& c, uint32_t items, uint32_t tiles_per_warp, cudaStream_t s) {
-    // down, whose K is short (eight groups at ffn 512), is bound by instruction issue: four groups per stage halve
-    // its per-stage bookkeeping (three stages still fit beside its small row tile).
-    if constexpr (BITS == 4 && NMAT == 1 && KS == 1) {
-        if ((c.F / 64) % 4 == 0) return launch_expert_ch<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, 4>(m, c, items, tiles_per_warp, s);
-    }
-    return launch_expert_ch<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, 2>(m, c, items, tiles_per_warp, s);
-}
-
-template <int NMAT, int KS, bool META_F16, int MW>
-int dispatch_bits(zc_moe* m, const Call& c, uint32_t items, uint32_t tpw, bool split, uint32_t bits, bool fold, cudaStream_t s) {
-    if (bits == 4) {
-        if (fold) return split ? launch_expert<4, true, NMAT, KS, true, META_F16, MW>(m, c, items, tpw, s) : launch_expert<4, false, NMAT, KS, true, META_F16, MW>(m, c, items, tpw, s);
-        return split ? launch_expert<4, true, NMAT, KS, false, META_F16, MW>(m, c, items, tpw, s) : launch_expert<4, false, NMAT, KS, false, META_F16, MW>(m, c, items, tpw, s);
-    }
-    return split ? launch_expert<8, true, NMAT, KS, false, META_F16, MW>(m, c, items, tpw, s) : launch_expert<8, false, NMAT, KS, false, META_F16, MW>(m, c, items, tpw, s);
-}
-template <int NMAT, int KS, int MW = 1>
-int dispatch_expert(zc_moe* m, const Call& c, uint32_t items, uint32_t tpw, bool split, uint32_t bits, bool fold, cudaStream_t s) {
-    return c.meta_f16 ? dispatch_bits<NMAT, KS, true, MW>(m, c, items, tpw, split, bits, fold, s)
-                      : dispatch_bits<NMAT, KS, false, MW>(m, c, items, tpw, split, bits, fold, s);
+template <int NMAT>
+int dispatch_expert(zc_moe* m, const Call& c, const StreamPlan& p, bool split, uint32_t bits, bool fold, cudaStream_t s) {
+    if (bits == 8) return c.meta_f16 ? dispatch_split<8, false, true, NMAT>(m, c, p, split, s) : dispatch_split<8, false, false, NMAT>(m, c, p, split, s);
+    if (fold) return c.meta_f16 ? dispatch_split<4, true, true, NMAT>(m, c, p, split, s) : dispatch_split<4, true, false, NMAT>(m, c, p, split, s);
+    return c.meta_f16 ? dispatch_split<4, false, true, NMAT>(m, c, p, split, s) : dispatch_split<4, false, false, NMAT>(m, c, p, split, s);
 }
 
 }  // namespace
+
+// TMA views of a layer's records (codes of gate and up together: the two projections have one geometry and lie one
+// projection apart; codes of down), encoded once when the handle is created.
+int make_stream_maps(zc_moe* m, LayerMem& L) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Encode encode = nullptr;
+    if (!encode) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q);
+        if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !p) return fail(m, ZC_EEXEC, "cuTensorMapEncodeTiled is not available");
+        encode = reinterpret_cast<Encode>(p);
+    }
+    auto make = [&](StreamMap& to, uint8_t* record, const Projection& pr, uint64_t pair_stride, uint32_t experts, uint64_t stride) {
+        const uint64_t row = uint64_t(pr.K) * pr.bits / 8;
+        const cuuint64_t dims[4] = {row, pr.N, pair_stride ? 2u : 1u, experts};
+        const cuuint64_t strides[3] = {row, pair_stride ? pair_stride : row * pr.N, stride};
+        const cuuint32_t box[4] = {128, pair_stride ? 16u : 32u, pair_stride ? 2u : 1u, 1}, elem[4] = {1, 1, 1, 1};
+        return encode(&to.m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, record + pr.codes, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    const zc_moe_desc& d = m->d;
+    const Projection gate = projection_of(d, 0), up = projection_of(d, 1), down = projection_of(d, 2);
+    bool ok = make(L.map_gate_up, L.records, gate, up.codes - gate.codes, d.local_experts, d.record_stride) &&
+              make(L.map_down, L.records, down, 0, d.local_experts, d.record_stride);
+    L.map_shared_gate_up = L.map_gate_up;
+    L.map_shared_down = L.map_down;
+    if (ok && d.has_shared) {
+        const zc_moe_desc sd = shared_desc_of(d);
+        const Projection sg = projection_of(sd, 0), su = projection_of(sd, 1), sdn = projection_of(sd, 2);
+        const uint64_t stride = (record_bytes_of(sd) + 16383) / 16384 * 16384;
+        ok = make(L.map_shared_gate_up, L.shared_record, sg, su.codes - sg.codes, 1, stride) && make(L.map_shared_down, L.shared_record, sdn, 0, 1, stride);
+    }
+    m->stream_maps = m->stream_maps && ok;      // a geometry TMA cannot describe stays with the item kernels
+    return ZC_OK;
+}
 
 static int launch_experts_decode_one(zc_moe* m, const Call& c, cudaStream_t s);
 
@@ -651,35 +825,56 @@ int launch_experts_decode(zc_moe* m, const Call& c, cudaStream_t s) {
     return total + n;
 }
 
+static bool stream_plan(const zc_moe* m, const Call& c, int nmat, bool split, uint32_t bits, StreamPlan& p) {
+    const uint32_t K = nmat == 2 ? c.H : c.F;
+    p.pairs = (K / 64 + (bits == 4 ? 7 : 3)) / (bits == 4 ? 8 : 4);
+    auto fits = [&]() { return stream_smem(p, split, K, bits) <= STREAM_SMEM_MAX; };
+    p.warps = MAX_WARPS; p.ks = 1; p.nbuf = 2;
+    if (!fits()) p.nbuf = 1;
+    // Four warps share a gate/up tile for the shortest batches (one tile per warp would leave most of the SMs without work) and
+    // where only one row block fits (hidden above 2560): there the warps of a CTA meet at every pass, and with a quarter of
+    // the tiles in flight they arrive closer together (256 tokens at hidden 4096: 492 us against 511 for the layer).
+    if (nmat == 2 && p.pairs >= 4 && (p.nbuf == 1 || c.T * (c.K + (c.has_shared ? 1 : 0)) <= 64)) p.ks = 4;
+    if (!fits()) p.ks = 1;
+    while (!fits() && p.warps > 4) p.warps /= 2;
+    p.rt = p.warps / p.ks; p.ks_shift = p.ks == 4 ? 2 : 0;
+    p.tiles_per_pass = nmat == 2 ? c.F / 16 : c.H / 32;
+    p.own = (c.E + p.warps * 32 - 1) / (p.warps * 32);
+    p.inv_tiles = 1.0f / float(p.tiles_per_pass); p.inv_grid = 1.0f / float(sm_count(m));
+    return fits();
+}
+
+// Batches that stay with the item kernels (csrc/experts_item.cu), whose many small CTAs start faster:
+//  - at most 20 rows: one or two tokens, all latency (1 / 2 tokens of 512 experts: 26.5 / 35.5 us a layer against 30.5 / 37.8);
+//  - where the tiles fill the streaming kernel's warps more than once but less than about twice, so that its second round is
+//    partly empty (12 / 16 tokens: 71.1 / 77.4 us against 72.9 / 81.6; 8 and 20 tokens: 60.4 and 101.5 against 58.4 and 98.5;
+//    hidden 2560, ffn 640: 8 / 12 tokens 76.4 / 96.2 against 82.2 / 97.6, 16 tokens 114 against 117). With hidden 4096 the
+//    item kernels have one CTA per SM and lose from two tokens on. The number of distinct experts is estimated for rows that
+//    fall evenly.
+static bool item_kernels_pay(const zc_moe* m, const Call& c) {
+    const double rows = double(c.T) * c.K, experts = c.local_experts;
+    if (rows <= 20) return true;
+    if (c.H > 2560 || c.item_rows_max) return false;
+    const double passes = experts * (1.0 - std::exp(-rows / experts)) + (c.has_shared ? (c.T + NROW - 1) / NROW : 0);
+    const double rounds = passes * (c.F / 16) / (double(sm_count(m)) * MAX_WARPS);
+    return rounds > 1.2 && rounds < 2.1;
+}
+
 static int launch_experts_decode_one(zc_moe* m, const Call& c, cudaStream_t s) {
-    const uint32_t routed = c.T * c.K < c.local_experts ? c.T * c.K : c.local_experts;
-    const uint32_t items = routed + (c.has_shared ? (c.T + NTOK - 1) / NTOK : 0);
     // A BF16 activation is exact as one FP16 term; an FP32 activation needs two, except under the
     // reference arithmetic, whose FP32 buffers hold BF16 values by contract.
     const bool split_x = c.act_dtype == ZC_F32 && !c.ref;
     // The SwiGLU rows h are FP32 in memory. By default the down product reads them as one FP16 term (11 significant
     // bits, against the 8 of the BF16 the reference rounds h to; measured 1.2e-3 x RMS max-abs at 64 tokens, inside the
-    // 2e-3 bound); with the "exact_h" option as two FP16 terms, which costs a second MMA per fragment (73 us against
-    // 56 us for the down launch of the benchmark layer). The reference arithmetic's h is BF16: exact in one term.
+    // 2e-3 bound); with the "exact_h" option as two FP16 terms, which costs a second MMA per fragment.
+    // The reference arithmetic's h is BF16: exact in one term.
     const bool split_h = !c.ref && m->exact_h;
-    const bool fold = m->fold_q4;
-    // Few rows in flight: split K over all eight warps so that even one token fills the machine.
-    const bool small = c.T * (c.K + (c.has_shared ? 1 : 0)) <= 64;
+    StreamPlan gate_up{}, down{};
+    if (!m->stream_maps || item_kernels_pay(m, c) || !stream_plan(m, c, 2, split_x, c.gate.bits, gate_up) || !stream_plan(m, c, 1, split_h, c.down.bits, down))
+        return launch_experts_item(m, c, s);
     int rc;
-    if (small) rc = dispatch_expert<2, 8>(m, c, items, 1, split_x, c.gate.bits, fold, s);
-#ifndef ZC_TPW_GU
-#define ZC_TPW_GU 2
-#endif
-#ifndef ZC_TPW_DN
-#define ZC_TPW_DN 4
-#endif
-    // As the few-row side of a long batch only a fraction of the items has work (the others leave at once): fewer
-    // tiles per warp, i.e. more and shorter CTAs per item, keep the SMs filled.
-    else rc = dispatch_expert<2, 1>(m, c, items, c.item_rows_max ? m->few_tiles_gate_up : ZC_TPW_GU, split_x, c.gate.bits, fold, s);
-    if (rc < 0) return rc;
-    if (small) rc = dispatch_expert<1, 2>(m, c, items, 1, split_h, c.down.bits, fold, s);
-    else rc = dispatch_expert<1, 1>(m, c, items, c.item_rows_max ? m->few_tiles_down : ZC_TPW_DN, split_h, c.down.bits, fold, s);
-    if (rc < 0) return rc;
+    if ((rc = dispatch_expert<2>(m, c, gate_up, split_x, c.gate.bits, m->fold_q4, s)) < 0) return rc;
+    if ((rc = dispatch_expert<1>(m, c, down, split_h, c.down.bits, m->fold_q4, s)) < 0) return rc;
     return 2;
 }
 
