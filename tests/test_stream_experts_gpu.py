@@ -25,7 +25,6 @@ TOL = 2e-3          # max-abs error over the output's RMS, the specification's b
     (5000, dict(hidden=128, ffn=128, experts=32, top_k=8, act_dtype=F32)),   # 5,600 passes: more than a table of 32 per CTA
     (45, dict(hidden=2048, experts=64, down_bits=8, q8_signed=1)),
     (45, dict(hidden=640, ffn=128, experts=32, gate_bits=8, up_bits=8, down_bits=8)),
-    (30, dict(hidden=2048, experts=64, gate_bits=8, up_bits=8, down_bits=4)),
     (64, dict(hidden=2560, ffn=640, experts=64, meta_dtype=BF16, act_dtype=F32, router_dtype=BF16, arith=ARITH_REFERENCE)),
 ])
 def test_streamed_experts_against_the_checker(tokens, kw):
@@ -41,8 +40,6 @@ def test_streamed_experts_against_the_checker(tokens, kw):
     w, gate = synth.router(cfg, SEED, 0), synth.shared_gate(cfg, SEED, 0)
     m.load_layer(0, np.stack(records), router_w=w, shared_record=shared, shared_gate_w=gate)
     x = synth.activations(cfg, SEED, 0, tokens)
-    if cfg.gate_bits > cfg.down_bits:
-        x = x / 16          # the generator's 8-bit weights reach 2.5: keeps the SwiGLU rows inside the 4-bit down projection's range (4094)
     dev = torch.from_numpy(x).to(device="cuda", dtype=m.act_torch)
     got = m.decode(0, dev)
     assert m.status() == 0
