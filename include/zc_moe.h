@@ -290,6 +290,8 @@ int zc_moe_stack_host(zc_moe* moe, const void* x_host, uint32_t tokens, void* ou
  *   0 selects the earlier per-group-drain kernel.
  *   "prefill_small_rows" (default 16, 0..64): in a long batch, experts with at most this many rows run on the streaming
  *   kernels and the grouped GEMM takes the others (0: the grouped GEMM takes every expert).
+ *   "expert_kernels" (default 0): which kernels run the decode family's experts: 0 by the batch, 1 the item kernels, 2 the
+ *   streaming kernels (ZC_EINVAL from a call whose shape they do not take). The two differ in the order of FP32 sums.
  *   "few_tiles_gate_up" (default 1), "few_tiles_down" (default 2), 1..4: 16-row tiles per warp of the item kernels in such
  *   launches; "meta_blocks" (default 1): the item kernels fetch scales and biases eight groups at a time (16-byte copies)
  *   for gate/up at hidden >= 4096; 2 does so wherever the layout allows, 3 uses four-group blocks for gate/up, 0 never

@@ -61,3 +61,67 @@ def test_a_token_does_not_depend_on_its_place_in_the_batch():
     x = torch.from_numpy(synth.activations(cfg, SEED, 0, 200)).to(device="cuda", dtype=torch.bfloat16)
     order = torch.from_numpy(np.random.default_rng(3).permutation(200)).cuda()
     assert torch.equal(m.decode(0, x)[order], m.decode(0, x[order].contiguous()))
+
+
+def expert_rows_against_64_bits(kw, kernels, fold=1, bias_only=False, rows=1024):
+    """(relative 2-norm error of the expert products of 32 experts with two-term SwiGLU rows, the handle's status)."""
+    import torch
+    from zerocool_b200.moe import Moe
+    from zerocool_b200.records import build_record, dequantise, float_to_meta, meta_to_float
+    base = dict(hidden=2048, ffn=512, experts=64, top_k=8, layers=1, local_experts=32, meta_dtype=F16, act_dtype=BF16, out_dtype=F32, max_tokens=64, q8_signed=1)
+    base.update(kw)
+    cfg = MoeConfig(**base)
+    rng = np.random.default_rng(5)
+    records = []
+    for e in range(32):
+        parts = []
+        for p in range(3):
+            codes, scales, _ = synth.projection_parts(cfg, SEED, 0, e, p)
+            s = meta_to_float(scales, cfg.meta_dtype)
+            if bias_only:
+                s, b = np.zeros_like(s), rng.uniform(0.01, 0.03, size=s.shape)
+            else:
+                b = (-8.0 if cfg.bits(p) == 4 else 0.0) * s + rng.uniform(-0.03, 0.03, size=s.shape)
+            parts.append((codes, float_to_meta(s.astype(np.float32), cfg.meta_dtype).reshape(scales.shape), float_to_meta(b.astype(np.float32), cfg.meta_dtype).reshape(scales.shape)))
+        records.append(build_record(cfg, parts))
+    m = Moe(cfg, 0)
+    m.load_layer(0, np.stack(records))
+    m.set_option("exact_h", 1)
+    m.set_option("fold_q4", fold)
+    m.set_option("expert_kernels", kernels)
+    x = torch.from_numpy(rng.standard_normal((rows, cfg.hidden)).astype(np.float32)).cuda()
+    x = (x.abs() * 0.05 if bias_only else x).to(m.act_torch)
+    ids = torch.arange(rows, device="cuda", dtype=torch.int32) % 32
+    y = m.ep_experts(0, x, ids).double()
+    error = norm = 0.0
+    for e in range(32):
+        w = [torch.from_numpy(dequantise(cfg, records[e], p)).cuda() for p in range(3)]
+        mine = x[ids == e].double()
+        gate = mine @ w[0].T
+        want = (gate * torch.sigmoid(gate) * (mine @ w[1].T)) @ w[2].T
+        error += float(((y[ids == e] - want) ** 2).sum())
+        norm += float((want ** 2).sum())
+    return (error / norm) ** 0.5, m.status()
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(act_dtype=F32), dict(gate_bits=8, up_bits=8, down_bits=8)])
+def test_bias_terms_keep_the_group_sums_24_bits(kw):
+    """Scales of zero leave the sums of bias x group sum, here all of one sign, so that every rounding shows. Each of the three
+    products may lose one step of 2^-23 of a partial sum over eight groups (the tensor core's adder) and half of one in each FP32
+    addition: on average below 2^-23 together. Group sums cut to 22 bits and added in the tensor core lose two to four times that."""
+    pytest.importorskip("torch")
+    error, status = expert_rows_against_64_bits(kw, 2, bias_only=True)
+    assert status == 0
+    assert error <= 3 * 2.0 ** -23, error
+
+
+@pytest.mark.parametrize("kw,fold", [(dict(act_dtype=F32), 1), (dict(), 0), (dict(act_dtype=F32), 0), (dict(hidden=2560, ffn=640, meta_dtype=BF16), 0),
+                                     (dict(gate_bits=8, up_bits=8, down_bits=8), 0)])
+def test_streaming_kernels_are_as_close_to_64_bits_as_the_item_kernels(kw, fold):
+    """Both accumulate the same products. The error is that of a few thousand group sums (1,024 rows x 8 groups of down, with
+    heavy-tailed rows): 8 % covers its scatter."""
+    pytest.importorskip("torch")
+    stream, status = expert_rows_against_64_bits(kw, 2, fold)
+    item, item_status = expert_rows_against_64_bits(kw, 1, fold)
+    assert status == 0 and item_status == 0
+    assert stream <= 1.08 * item, (stream, item)

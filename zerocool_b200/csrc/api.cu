@@ -898,6 +898,13 @@ int zc_moe_set_option(zc_moe* m, const char* name, int value) {
         m->prefill_small_rows = uint32_t(value);
         return ZC_OK;
     }
+    if (!std::strcmp(name, "expert_kernels")) {
+        if (value < 0 || value > 2) return fail(m, ZC_EINVAL, "expert_kernels must be 0..2");
+        DeviceGuard guard(m->device);
+        drop_graphs(m);
+        m->expert_kernels = uint32_t(value);
+        return ZC_OK;
+    }
     if (!std::strcmp(name, "few_tiles_gate_up") || !std::strcmp(name, "few_tiles_down")) {
         if (value < 1 || value > 4) return fail(m, ZC_EINVAL, "few_tiles_* must be 1..4");
         DeviceGuard guard(m->device);

@@ -275,6 +275,7 @@ struct zc_moe {
     uint32_t prefill_small_rows = 16;   // long batches: experts with at most this many rows run on the streaming kernels (0 = none)
     bool prefill_wide = true;     // long batches: wide-tile kernel with accumulators resident in TMEM (false: per-group drain kernel)
     bool fold_q4 = true;          // Q4 codes enter the MMA with their 1024 offset (removed from the FP32 group sum)
+    uint32_t expert_kernels = 0;  // decode family: 0 by the rule in experts_decode.cu, 1 item kernels, 2 streaming kernels
     bool stream_maps = true;      // the records' geometry has TMA views (make_stream_maps)
     bool profiling = false;
     struct Span { int kind; cudaEvent_t start, stop; };

@@ -25,8 +25,13 @@
 //    a product of its own:
 //        acc += scale[row, g] * sum_k(q * x);     acc += bias[row, :] . group sums of x
 //    which is the reference's affine_dot form (qwen.metal:46-62) with an exact inner sum. The bias product is an
-//    m16n8k4 TF32 MMA over four groups: a 16-bit bias is exact in TF32, and the FP32 group sum enters as two TF32 terms
-//    (22 significant bits), so it replaces two conversions and four FMAs per group and 16 x 8 tile by a fraction of an MMA.
+//    TF32 MMA over a pair of stages (eight Q4 or four Q8 groups): a 16-bit bias is exact in TF32, and the FP32 group sum enters
+//    as three TF32 terms, all of its 24 bits, smallest term first. It has accumulators of its own, which are added to acc in
+//    FP32: the MMA's adder does not round to nearest, and in acc it would do so once per product. The product stands
+//    between the two stages of its pair, where it cancels against the codes' part soonest. Error against 64 bits beside the item
+//    kernels' FMA per group (two-term rows): gate/up 8.3e-6 / 8.3e-6 and down 2.26e-5 / 2.30e-5 (folded Q4), 2.29e-7 / 2.31e-7
+//    and 3.7e-7 / 4.2e-7 (not folded), a Q8 layer 2.8e-7 / 3.1e-7; biases alone 1.9e-7 / 2.0e-7, and 1.3e-7 / 0.5e-7 where all
+//    terms have one sign.
 //  * Q4 codes become FP16 with one logic operation per two weights: (w & 0x000f000f) | 0x6400 is the
 //    half2 (1024+q_lo, 1024+q_hi), and (w & 0x00f000f0) | 0x6400 is (1024+16 q, 1024+16 q). With FOLD
 //    those values go into the MMA as they are: the activations that meet a "q" slot are staged multiplied by 16
@@ -100,6 +105,14 @@ __device__ __forceinline__ void mma_tf32_1688(float (&d)[4], float a0, float a1,
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+
+// v as three TF32 values (11 + 11 + 2 significant bits: exact).
+__device__ __forceinline__ void tf32_terms(float v, float& h, float& m, float& l) {
+    h = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+    const float r = v - h;
+    m = __uint_as_float(__float_as_uint(r) & 0xffffe000u);
+    l = r - m;
 }
 
 // How a launch is cut (chosen on the host, stream_plan): warps per CTA, warps that share a row tile, staged passes,
@@ -185,30 +198,29 @@ __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, RowOf 
         // accumulated result is multiplied by 1/16 (exact) when it is finished.
         constexpr float EVEN = (FOLD && Q4ORDER) ? 16.0f : 1.0f;
         constexpr int order_q4[8] = {0, 4, 1, 5, 2, 6, 3, 7};
-        uint32_t ph[4], pl[4];
-        float even = 0.0f, odd = 0.0f;         // sums of the values as fed to the MMA
+        alignas(16) __half2 h[4], l[4];
+        float sf = 0.0f, sn = 0.0f;            // sums of the values as fed to the MMA, k ascending: as staged, and in natural scale
+        float fed[8];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int a = Q4ORDER ? order_q4[2 * i] : 2 * i, b = Q4ORDER ? order_q4[2 * i + 1] : 2 * i + 1;
             const float va = (a & 1) ? v[a] : v[a] * EVEN, vb = (b & 1) ? v[b] : v[b] * EVEN;
             most = fmaxf(most, fmaxf(fabsf(va), fabsf(vb)));
-            const __half2 h = __floats2half2_rn(va, vb);
-            ph[i] = *reinterpret_cast<const uint32_t*>(&h);
-            float2 fed = __half22float2(h);
+            h[i] = __floats2half2_rn(va, vb);
+            float2 f = __half22float2(h[i]);
             if (SPLIT) {
-                const __half2 l = __floats2half2_rn(va - fed.x, vb - fed.y);
-                pl[i] = *reinterpret_cast<const uint32_t*>(&l);
-                const float2 low = __half22float2(l);
-                fed.x += low.x; fed.y += low.y;
+                l[i] = __floats2half2_rn(va - f.x, vb - f.y);
+                const float2 low = __half22float2(l[i]);
+                f.x += low.x; f.y += low.y;
             }
-            if (a & 1) odd += fed.x; else even += fed.x;
-            if (b & 1) odd += fed.y; else even += fed.y;
+            fed[a] = f.x; fed[b] = f.y;
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { sf += fed[i]; sn += (i & 1) ? fed[i] : fed[i] * (1.0f / EVEN); }
         // The bias term multiplies the sum of the activations. Outside the reference arithmetic it uses the sum of
         // the values the MMA really sees, so that a rounding of an activation to FP16 enters the result through the
         // weight s q + b and not through s q alone.
-        if (!ref) sx = even * (1.0f / EVEN) + odd;
-        float sf = even + odd;
+        if (!ref) sx = sn;
 #pragma unroll
         for (int off = 1; off <= 4; off <<= 1) {
             sx += __shfl_xor_sync(0xffffffffu, sx, off);
@@ -222,8 +234,8 @@ __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, RowOf 
                     o[0] = o[2] = -1024.0f * sf;
                 }
             }
-            *reinterpret_cast<uint4*>(hi + n * RS + q * 8) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-            if (SPLIT) *reinterpret_cast<uint4*>(lo + n * RS + q * 8) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+            *reinterpret_cast<uint4*>(hi + n * RS + q * 8) = *reinterpret_cast<const uint4*>(h);
+            if (SPLIT) *reinterpret_cast<uint4*>(lo + n * RS + q * 8) = *reinterpret_cast<const uint4*>(l);
         }
         piece += stride;
     }
@@ -269,7 +281,8 @@ __device__ __forceinline__ void dequant_q8(uint32_t w, bool is_signed, uint32_t 
 }
 
 // d[m] (16 rows x 8 tokens) = off + sum over one 64-wide group of code * x, for the two 16-row fragments m of a stage (the
-// lane's rows g: w[m][0], g+8: w[m][1]). The fragments' independent MMA chains are interleaved.
+// lane's rows g: w[m][0], g+8: w[m][1]). The fragments' independent MMA chains are interleaved. The low terms of a word follow its high
+// terms, as in the item kernels: the adder drops bits relative to the running sum, which the high terms bring down from the folded offset.
 template <int BITS, bool SPLIT, bool FOLD>
 __device__ __forceinline__ void group_mma(float (&d)[2][4], const float4& off, const uint32_t (&w)[2][2][BITS / 2],
                                           const uint4 (&bh)[2], const uint4 (&bl)[2], bool q8_signed) {
@@ -285,18 +298,18 @@ __device__ __forceinline__ void group_mma(float (&d)[2][4], const float4& off, c
                 else dequant_q8(w[m][r][i], q8_signed, p[m][r]);
             }
 #pragma unroll
-        for (int h = 0; h < PER; ++h) {
-            const int step = i * PER + h;                                  // of the group's four
-            const uint4 hi = bh[step / 2], lo = bl[step / 2];
-            const uint32_t b0 = step % 2 ? hi.z : hi.x, b1 = step % 2 ? hi.w : hi.y;
+        for (int t = 0; t < (SPLIT ? 2 : 1); ++t)                          // the low terms after the word's high terms
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-                if (step == 0) mma_f16_16816_c(d[m], p[m][0][0], p[m][1][0], p[m][0][1], p[m][1][1], b0, b1, off.x, off.y, off.z, off.w);
-                else mma_f16_16816(d[m], p[m][0][2 * h], p[m][1][2 * h], p[m][0][2 * h + 1], p[m][1][2 * h + 1], b0, b1);
-                if constexpr (SPLIT)
-                    mma_f16_16816(d[m], p[m][0][2 * h], p[m][1][2 * h], p[m][0][2 * h + 1], p[m][1][2 * h + 1], step % 2 ? lo.z : lo.x, step % 2 ? lo.w : lo.y);
+            for (int h = 0; h < PER; ++h) {
+                const int step = i * PER + h;                              // of the group's four
+                const uint4 v = t ? bl[step / 2] : bh[step / 2];
+                const uint32_t b0 = step % 2 ? v.z : v.x, b1 = step % 2 ? v.w : v.y;
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    if (step == 0 && t == 0) mma_f16_16816_c(d[m], p[m][0][0], p[m][1][0], p[m][0][1], p[m][1][1], b0, b1, off.x, off.y, off.z, off.w);
+                    else mma_f16_16816(d[m], p[m][0][2 * h], p[m][1][2 * h], p[m][0][2 * h + 1], p[m][1][2 * h + 1], b0, b1);
+                }
             }
-        }
     }
 }
 
@@ -586,6 +599,37 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) stream_kernel(const Call c, co
                         const __half* xb = xhi + row_at * RS + pair * (2 * GPS * 64) + cq * 16;
 #pragma unroll
                         for (int half = 0; half < 2; ++half) {
+                            if (half == 1) {         // the bias product of the pair's groups
+                                const float* sp = sx + row_at * GP + pair * (2 * GPS);
+                                float add[2][4] = {};
+                                if constexpr (BITS == 4) {           // k slots cq and cq + 4 of the MMA are groups 2 cq and 2 cq + 1
+                                    const float2 v = *reinterpret_cast<const float2*>(sp + 2 * cq);
+                                    float h0, m0, l0, h1, m1, l1;
+                                    tf32_terms(v.x, h0, m0, l0);
+                                    tf32_terms(v.y, h1, m1, l1);
+#pragma unroll
+                                    for (int m = 0; m < 2; ++m) {
+                                        const float2 b0 = meta_pair<META_F16>(bi[m][0]), b1 = meta_pair<META_F16>(bi[m][1]);
+                                        mma_tf32_1688(add[m], b0.x, b1.x, b0.y, b1.y, l0, l1);
+                                        mma_tf32_1688(add[m], b0.x, b1.x, b0.y, b1.y, m0, m1);
+                                        mma_tf32_1688(add[m], b0.x, b1.x, b0.y, b1.y, h0, h1);
+                                    }
+                                } else {                             // k slot cq is group cq
+                                    float h0, m0, l0;
+                                    tf32_terms(sp[cq], h0, m0, l0);
+#pragma unroll
+                                    for (int m = 0; m < 2; ++m) {
+                                        const float b0 = meta_pair<META_F16>(bi[m][0]).x, b1 = meta_pair<META_F16>(bi[m][1]).x;
+                                        mma_tf32_1684(add[m], b0, b1, l0);
+                                        mma_tf32_1684(add[m], b0, b1, m0);
+                                        mma_tf32_1684(add[m], b0, b1, h0);
+                                    }
+                                }
+#pragma unroll
+                                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) acc[m][i] += add[m][i];
+                            }
                             if (half == 0 || pair * 2 + 1 < stages) {
                                 wait_bar(bar_base + half * 8, half ? parity1 : parity0);
                                 if (half) parity1 ^= 1; else parity0 ^= 1;
@@ -621,27 +665,6 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) stream_kernel(const Call c, co
                                         const float s0 = j % 2 ? p0.y : p0.x, s1 = j % 2 ? p1.y : p1.x;
                                         acc[m][0] = __fmaf_rn(s0, d[m][0], acc[m][0]); acc[m][1] = __fmaf_rn(s0, d[m][1], acc[m][1]);
                                         acc[m][2] = __fmaf_rn(s1, d[m][2], acc[m][2]); acc[m][3] = __fmaf_rn(s1, d[m][3], acc[m][3]);
-                                    }
-                                }
-                            }
-                            if (half == 1) {         // the bias product of the pair's groups
-                                const float* sp = sx + row_at * GP + pair * (2 * GPS);
-                                if constexpr (BITS == 4) {           // k slots cq and cq + 4 of the MMA are groups 2 cq and 2 cq + 1
-                                    const float2 v = *reinterpret_cast<const float2*>(sp + 2 * cq);
-                                    const float h0 = __uint_as_float(__float_as_uint(v.x) & 0xffffe000u), h1 = __uint_as_float(__float_as_uint(v.y) & 0xffffe000u);
-#pragma unroll
-                                    for (int m = 0; m < 2; ++m) {
-                                        const float2 b0 = meta_pair<META_F16>(bi[m][0]), b1 = meta_pair<META_F16>(bi[m][1]);
-                                        mma_tf32_1688(acc[m], b0.x, b1.x, b0.y, b1.y, h0, h1);
-                                        mma_tf32_1688(acc[m], b0.x, b1.x, b0.y, b1.y, v.x - h0, v.y - h1);
-                                    }
-                                } else {                             // k slot cq is group cq
-                                    const float v = sp[cq], h = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-#pragma unroll
-                                    for (int m = 0; m < 2; ++m) {
-                                        const float b0 = meta_pair<META_F16>(bi[m][0]).x, b1 = meta_pair<META_F16>(bi[m][1]).x;
-                                        mma_tf32_1684(acc[m], b0, b1, h);
-                                        mma_tf32_1684(acc[m], b0, b1, v - h);
                                     }
                                 }
                             }
@@ -870,8 +893,9 @@ static int launch_experts_decode_one(zc_moe* m, const Call& c, cudaStream_t s) {
     // The reference arithmetic's h is BF16: exact in one term.
     const bool split_h = !c.ref && m->exact_h;
     StreamPlan gate_up{}, down{};
-    if (!m->stream_maps || item_kernels_pay(m, c) || !stream_plan(m, c, 2, split_x, c.gate.bits, gate_up) || !stream_plan(m, c, 1, split_h, c.down.bits, down))
-        return launch_experts_item(m, c, s);
+    const bool fits = m->stream_maps && stream_plan(m, c, 2, split_x, c.gate.bits, gate_up) && stream_plan(m, c, 1, split_h, c.down.bits, down);
+    if (m->expert_kernels == 2 && !fits) return fail(m, ZC_EINVAL, "expert_kernels = 2: the streaming kernels do not take this shape");
+    if (m->expert_kernels == 1 || !fits || (m->expert_kernels == 0 && item_kernels_pay(m, c))) return launch_experts_item(m, c, s);
     int rc;
     if ((rc = dispatch_expert<2>(m, c, gate_up, split_x, c.gate.bits, m->fold_q4, s)) < 0) return rc;
     if ((rc = dispatch_expert<1>(m, c, down, split_h, c.down.bits, m->fold_q4, s)) < 0) return rc;
