@@ -139,7 +139,7 @@ int run_layer(zc_moe* m, uint32_t layer, const void* x, uint32_t tokens, void* o
     if (family < 0) family = (tokens >= 64 && uint64_t(tokens) * m->d.top_k >= 24ull * m->d.local_experts) ? 1 : 0;
     if (family == 1 && !m->pf_tiles) family = 0;      // formats the prefill kernels do not take, or a decode-sized handle
     int n, total = 0;
-    if ((n = launch_router_partial(m, c, s)) < 0) return n; total += n;
+    if ((n = launch_router(m, c, s)) < 0) return n; total += n;
     if ((n = launch_route_permute(m, c, s, true, true)) < 0) return n; total += n;
     if ((n = launch_experts(m, c, s, family)) < 0) return n; total += n;
     if (hc) n = launch_combine_hc(m, c, hc->hyper, hc->inject, hc->out, s);
@@ -169,6 +169,17 @@ int zc_moe_desc_finalize(zc_moe_desc* d) {
     for (int p = 0; p < 3; ++p) { const Projection pr = projection_of(*d, p); bytes = pr.biases + uint64_t(pr.N) * (pr.K / d->group) * 2; }
     d->record_bytes = bytes;
     d->record_stride = (bytes + 16383) / 16384 * 16384;
+    return ZC_OK;
+}
+
+int zc_moe_kernel_choice(const zc_moe_desc* desc, uint32_t tokens, uint32_t sms, uint32_t choice[4]) {
+    if (!desc || !tokens || !sms || !choice) return fail(nullptr, ZC_EINVAL, "null descriptor or choice, or no tokens or SMs");
+    zc_moe_desc d = *desc;
+    if (!d.local_experts) d.local_experts = d.experts - d.first_expert;
+    std::string why;
+    if (validate_desc(d, why) != ZC_OK) return fail(nullptr, ZC_EINVAL, why);
+    const RouterCut cut = router_cut(tokens, d.experts, d.has_shared, sms);
+    choice[0] = cut.ranks; choice[1] = cut.tokens; choice[2] = choice[3] = 0;
     return ZC_OK;
 }
 
@@ -447,7 +458,7 @@ int zc_moe_forward_routed(zc_moe* m, uint32_t layer, const void* x, uint32_t tok
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Call c = make_call(m, layer, x, tokens, out);
     int n, total = 0;
-    if ((n = launch_router_partial(m, c, s)) < 0) return n; total += n;          // the scores of the recorded experts, and the shared gate
+    if ((n = launch_router(m, c, s)) < 0) return n; total += n;          // the scores of the recorded experts, and the shared gate
     if ((n = launch_forced_weights(m, c, ids, s)) < 0) return n; total += n;
     if ((n = launch_route_permute(m, c, s, false, true)) < 0) return n; total += n;
     const bool wide = tokens >= 64 && uint64_t(tokens) * m->d.top_k >= 24ull * m->d.local_experts && m->pf_tiles;
@@ -480,7 +491,7 @@ int zc_moe_ep_dispatch(zc_moe* m, uint32_t layer, const void* x, uint32_t tokens
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const Call c = make_call(m, layer, x, tokens, nullptr);
     int n, total = 0;
-    if ((n = launch_router_partial(m, c, s)) < 0) return n; total += n;
+    if ((n = launch_router(m, c, s)) < 0) return n; total += n;
     if ((n = launch_route_permute(m, c, s, true, true)) < 0) return n; total += n;
     if ((n = launch_ep_gather(m, c, rows, row_experts, s)) < 0) return n; total += n;
     m->launches += total;
@@ -545,7 +556,7 @@ int ep_ready(zc_moe* m, uint32_t layer) {
 int ep_send_phase(zc_moe* m, uint32_t layer, const void* x, uint32_t tokens, cudaStream_t s) {
     const Call c = make_call(m, layer, x, tokens, nullptr);
     int n, total = 0;
-    if ((n = launch_router_partial(m, c, s)) < 0) return n; total += n;
+    if ((n = launch_router(m, c, s)) < 0) return n; total += n;
     if ((n = launch_route_permute(m, c, s, true, true)) < 0) return n; total += n;
     if ((n = launch_ep_send(m, c, s)) < 0) return n; total += n;
     if (c.has_shared) {

@@ -285,7 +285,8 @@ struct zc_moe {
 namespace zc {
 // Launchers (each returns the number of kernels launched, or a negative ZC_* code with moe->error set).
 int launch_router(zc_moe* m, const Call& c, cudaStream_t s);
-int launch_router_partial(zc_moe* m, const Call& c, cudaStream_t s);
+struct RouterCut { uint32_t ranks, tokens; };     // CTAs that share the sixteen partitions of a tile; tokens of a tile
+RouterCut router_cut(uint32_t tokens, uint32_t experts, bool shared, uint32_t sms);
 int launch_route_permute(zc_moe* m, const Call& c, cudaStream_t s, bool do_route, bool do_permute);
 int launch_forced_weights(zc_moe* m, const Call& c, const int32_t* forced, cudaStream_t s);
 int launch_experts_decode(zc_moe* m, const Call& c, cudaStream_t s);

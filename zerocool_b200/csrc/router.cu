@@ -1,16 +1,16 @@
 // Router logits (and the shared-expert gate scalar) in fp32 with a pinned accumulation order.
 //
 // Replaces router_mm + router_accumulate (kernels/metal/qwen.metal:512-534, launched from
-// src/engine/metal.mm:818-822) and keeps their structure: K is cut into sixteen contiguous partitions,
-// each partition is a k-ascending chain of fused multiply-adds that one thread owns, the sixteen
-// partials go to memory as [16, T, rows], and they are added in order 0..15 by the last of the sixteen
-// partition CTAs of a tile to finish. The order is part of the contract
+// src/engine/metal.mm:818-822) and keeps their arithmetic: K is cut into sixteen contiguous partitions,
+// each partition is a k-ascending chain of fused multiply-adds that one thread owns, and the sixteen
+// partials are added in order 0..15, starting from zero. The order is part of the contract
 // because one last-bit change in a logit can flip a top-k decision; it reproduces the MLX bit patterns
 // the reference's own test holds (tests/test_qwen.cpp:798-826).
 //
-// router_partial_kernel (the entry point that may not allocate): grid (row tiles of 32, 16 partitions, token tiles). A CTA
-// stages its slice of x (k-major) and of the router rows (k-major) in shared memory, then every thread runs its chains.
-// Layer calls use router_cluster_kernel up to 128 tokens and router_tile_kernel beyond.
+// Layer calls use router_cluster_kernel up to 128 tokens and router_tile_kernel beyond (router_cut): their partials stay in
+// shared memory. router_partial_kernel serves the entry point that may not allocate: grid (row tiles of 32, 16 partitions, token
+// tiles); a CTA stages its slice of x (k-major) and of the router rows (k-major) in shared memory, every thread runs its chains,
+// the partials go to memory as [16, T, rows], and the last of the sixteen CTAs of a tile to finish adds them.
 #include "common.cuh"
 #include <cooperative_groups.h>
 
@@ -621,31 +621,40 @@ int launch_router_tile(zc_moe* m, const Call& c, uint32_t ranks, bool wide, cuda
 
 }  // namespace
 
-int launch_router_partial(zc_moe* m, const Call& c, cudaStream_t s) {
-    // Up to 128 tokens small cluster tiles win on latency: at 64 tokens, 544 CTAs of 16 tokens x 32 rows measured 19 us
-    // against 21 us (32 x 32) and 25 us (32 x 64, whose 144 large CTAs do not all find a cluster slot in the first wave).
-    int n = 0;
-    if (c.T <= 8) n = launch_router_cluster<8, 1>(m, c, s);
-    else if (c.T <= ZC_ROUTER_SMALL_T) n = launch_router_cluster<16, 1>(m, c, s);
-    if (n != 0) return n;
-    // Beyond, the register-tiled form. Splitting the partitions over eight CTAs pays unless the 64 x 64 tiles fill the SMs
-    // evenly: 256 tiles (2048 tokens, 512 experts) 142 us whole against 152 us split, 376 tiles 256 against 217, 72 tiles 90
-    // against 52; from 480 tiles on, tiles of twice the tokens (a third fewer shared-memory reads per product) 387 against
-    // 405 us at 6430 tokens. A device that cannot host a cluster of eight takes whole tiles.
-    const size_t tiles = size_t((c.T + 63) / 64) * ((c.E + RT_ROWS - 1) / RT_ROWS);
-    const bool f32x = c.act_dtype == ZC_F32, f32w = c.router_dtype == ZC_F32;
-    uint32_t ranks = tiles >= 480 || (tiles >= 240 && tiles <= 296) ? 1 : CLUSTER_SIZE;
-    for (;;) {
-        n = f32x ? (f32w ? launch_router_tile<true, true>(m, c, ranks, tiles >= 480, s) : launch_router_tile<true, false>(m, c, ranks, tiles >= 480, s))
-                 : (f32w ? launch_router_tile<false, true>(m, c, ranks, tiles >= 480, s) : launch_router_tile<false, false>(m, c, ranks, tiles >= 480, s));
-        if (n != 0) return n;
-        if (ranks == 1) return fail(m, ZC_EEXEC, "router: the device does not host the kernel");
-        ranks = 1;
-    }
+// How the router is cut. Up to 128 tokens small cluster tiles win on latency: at 64 tokens, 544 CTAs of 16 tokens x 32 rows
+// measured 19 us against 21 us (32 x 32) and 25 us (32 x 64, whose 144 large CTAs do not all find a cluster slot in the
+// first wave).
+// Beyond, the register-tiled form. Splitting the partitions over eight CTAs pays unless the 64 x 64 tiles, the shared gate's
+// row tile among them, fill the SMs twice and no more: whole tiles then take 141 us at hidden 2048 whatever their number, and
+// 198 as soon as one SM has a third one; split ones take 0.56 us a tile, the gate's about half of that. 512 experts and a shared one
+// (whole / split us): 1856 tokens, 261 tiles, 141 / 139; 1920, 270, 141 / 143; 2048, 288, 141 / 152; 2049, 297, 198 / 154; 2368, 333,
+// 200 / 173. Without the shared expert 2368 tokens, 296 tiles, 141 / 163; 128 experts and a shared one 8192 tokens, 384, 199 / 176.
+// From 480 tiles of experts on, tiles of twice the tokens (a third fewer shared-memory reads per product): 387 against 405 us at
+// 6430 tokens.
+RouterCut router_cut(uint32_t tokens, uint32_t experts, bool shared, uint32_t sms) {
+    if (tokens <= ZC_ROUTER_SMALL_T) return {uint32_t(CLUSTER_SIZE), tokens <= 8 ? 8u : 16u};
+    const uint64_t token_tiles = (tokens + 63) / 64, full = token_tiles * ((experts + RT_ROWS - 1) / RT_ROWS);
+    const uint64_t all = token_tiles * ((experts + shared + RT_ROWS - 1) / RT_ROWS);       // all - full: tiles of the gate's row alone
+    if (full >= 480) return {1, 128};
+    const bool twice = all <= 2ull * sms && 10 * full + 5 * (all - full) >= 17ull * sms;
+    return {twice ? 1u : uint32_t(CLUSTER_SIZE), 64};
 }
 
-// The router operator: one launch (partials, then the ordered sum by the last partition CTA of each tile).
-int launch_router(zc_moe* m, const Call& c, cudaStream_t s) { return launch_router_partial(m, c, s); }
+int launch_router(zc_moe* m, const Call& c, cudaStream_t s) {
+    const RouterCut cut = router_cut(c.T, c.E, c.has_shared, sm_count(m));
+    int n = 0;
+    if (cut.tokens == 8) n = launch_router_cluster<8, 1>(m, c, s);
+    else if (cut.tokens == 16) n = launch_router_cluster<16, 1>(m, c, s);
+    if (n != 0) return n;
+    // A device that cannot host a cluster of eight takes whole tiles.
+    const bool f32x = c.act_dtype == ZC_F32, f32w = c.router_dtype == ZC_F32, wide = cut.tokens == 128;
+    for (uint32_t ranks = cut.ranks;; ranks = 1) {
+        n = f32x ? (f32w ? launch_router_tile<true, true>(m, c, ranks, wide, s) : launch_router_tile<true, false>(m, c, ranks, wide, s))
+                 : (f32w ? launch_router_tile<false, true>(m, c, ranks, wide, s) : launch_router_tile<false, false>(m, c, ranks, wide, s));
+        if (n != 0) return n;
+        if (ranks == 1) return fail(m, ZC_EEXEC, "router: the device does not host the kernel");
+    }
+}
 
 }  // namespace zc
 

@@ -26,7 +26,7 @@ class Cancelled(RuntimeError):
     """The reference's "generation cancelled" (src/engine/model.cpp:15)."""
 
 EXPORTS = [
-    "zc_moe_desc_finalize", "zc_moe_create", "zc_moe_destroy", "zc_moe_last_error", "zc_last_error",
+    "zc_moe_desc_finalize", "zc_moe_kernel_choice", "zc_moe_create", "zc_moe_destroy", "zc_moe_last_error", "zc_last_error",
     "zc_moe_load_layer", "zc_moe_set_router_bias", "zc_moe_layer_buffers", "zc_moe_router", "zc_router_logits_noalloc", "zc_moe_route", "zc_moe_permute",
     "zc_moe_combine", "zc_activation_bf16", "zc_moe_decode", "zc_moe_prefill", "zc_moe_forward", "zc_moe_forward_routed", "zc_moe_hc_mix", "zc_moe_forward_hc", "zc_moe_ep_dispatch", "zc_moe_ep_experts", "zc_moe_ep_combine",
     "zc_moe_ep_export", "zc_moe_ep_attach", "zc_moe_ep_layer", "zc_moe_ep_send", "zc_moe_ep_process", "zc_moe_ep_finish", "zc_moe_ep_stack", "zc_moe_ep_stack_eager",
@@ -65,6 +65,7 @@ def load_library():
     lib = ctypes.CDLL(LIB_PATH)
     vp, u32, u64, i32 = ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int
     lib.zc_moe_desc_finalize.argtypes = [ctypes.POINTER(Desc)]
+    lib.zc_moe_kernel_choice.argtypes = [ctypes.POINTER(Desc), u32, u32, ctypes.POINTER(u32)]
     lib.zc_moe_create.argtypes = [ctypes.POINTER(Desc), i32, ctypes.POINTER(vp)]
     lib.zc_moe_destroy.argtypes = [vp]
     lib.zc_moe_destroy.restype = None
@@ -125,6 +126,16 @@ def make_desc(cfg: MoeConfig):
     for name, value in cfg.as_dict().items():
         setattr(d, name, int(value))
     return d
+
+
+def kernel_choice(cfg: MoeConfig, tokens, sms=148):
+    """``zc_moe_kernel_choice``: dict(router_ranks, router_tokens) of a layer call, by the library's rules."""
+    lib = load_library()
+    desc, choice = make_desc(cfg), (ctypes.c_uint32 * 4)()
+    rc = lib.zc_moe_kernel_choice(ctypes.byref(desc), int(tokens), int(sms), choice)
+    if rc != ZC_OK:
+        _raise(rc, lib.zc_last_error())
+    return dict(router_ranks=choice[0], router_tokens=choice[1])
 
 
 def _raise(code, text):
