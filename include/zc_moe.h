@@ -102,7 +102,8 @@ int zc_moe_desc_finalize(zc_moe_desc* desc);
 
 /* Which kernels the library's rules give a layer call of `tokens` tokens on a device with `sms` SMs (no device needed):
  * choice[0], [1] the router's cut: CTAs that share the K of a tile (8 or 1), tokens of a tile (8 or 16 up to 128 tokens, else
- * 64 or 128); choice[2], [3] 0. */
+ * 64 or 128); choice[2] the decode family's expert kernels, 1 item or 2 streaming (the values of the option "expert_kernels");
+ * choice[3] 0. */
 int zc_moe_kernel_choice(const zc_moe_desc* desc, uint32_t tokens, uint32_t sms, uint32_t choice[4]);
 
 /* Replaces Model::Model's Metal + Resident + ExpertCache construction for this path

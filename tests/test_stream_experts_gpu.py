@@ -125,3 +125,46 @@ def test_streaming_kernels_are_as_close_to_64_bits_as_the_item_kernels(kw, fold)
     item, item_status = expert_rows_against_64_bits(kw, 1, fold)
     assert status == 0 and item_status == 0
     assert stream <= 1.08 * item, (stream, item)
+
+
+@pytest.mark.parametrize("tokens,kernels", [(4, 1), (8, 2), (40, 2)])
+def test_the_shared_expert_alone_counts_no_routed_rows(tokens, kernels):
+    """A launch with an empty item list has the shared expert's passes only: a few tokens of it run on the item kernels, whatever
+    the layer's routed rows would be. The two kernels add in different orders, so equal bits tell which one ran."""
+    torch = pytest.importorskip("torch")
+    from zerocool_b200.moe import Moe
+    m = Moe(util.cfg2(experts=64, top_k=8, local_experts=32, max_tokens=64), 0)
+    m.synth_fill_layer(0, SEED)
+    x = torch.from_numpy(synth.activations(m.cfg, SEED, 0, tokens)).to(device="cuda", dtype=torch.bfloat16)
+    m.ep_dispatch(0, x)
+    y = torch.zeros(tokens * 8, m.cfg.hidden, device="cuda")
+    outs = []
+    for choice in (0, 1, 2):
+        m.set_option("expert_kernels", choice)
+        outs.append(m.ep_combine(0, x, y).clone())
+    assert m.status() == 0
+    assert not torch.equal(outs[1], outs[2])
+    assert torch.equal(outs[0], outs[kernels])
+
+
+def test_received_rows_are_counted_by_tokens_and_not_by_capacity():
+    """The owner step of expert parallelism: 128 local experts of a handle with room for 4 x 640 rows, one rank of 64 tokens
+    (640 rows expected: streaming) - and the same bits as the streaming kernels when they are named."""
+    torch = pytest.importorskip("torch")
+    from zerocool_b200.ep import attach_local, emulate_peer
+    from zerocool_b200.moe import Moe
+    parts = []
+    for r in range(4):
+        m = Moe(util.cfg2(first_expert=r * 128, local_experts=128, max_tokens=64), 0)
+        m.synth_fill_layer(0, SEED)
+        parts.append(m)
+    attach_local(parts)
+    xs = [torch.from_numpy(synth.activations(parts[0].cfg, SEED + r, 0, 64)).to(device="cuda", dtype=torch.bfloat16) for r in range(4)]
+    outs = {}
+    for choice in (0, 1, 2):
+        for m in parts:
+            m.set_option("expert_kernels", choice)
+        outs[choice] = [o.clone() for o in emulate_peer(parts, 0, xs)]
+    assert all(m.status() == 0 for m in parts)
+    assert any(not torch.equal(a, b) for a, b in zip(outs[1], outs[2]))
+    assert all(torch.equal(a, b) for a, b in zip(outs[0], outs[2]))

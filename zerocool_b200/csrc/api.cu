@@ -179,7 +179,14 @@ int zc_moe_kernel_choice(const zc_moe_desc* desc, uint32_t tokens, uint32_t sms,
     std::string why;
     if (validate_desc(d, why) != ZC_OK) return fail(nullptr, ZC_EINVAL, why);
     const RouterCut cut = router_cut(tokens, d.experts, d.has_shared, sms);
-    choice[0] = cut.ranks; choice[1] = cut.tokens; choice[2] = choice[3] = 0;
+    ExpertLoad l{};
+    l.rows = tokens * d.top_k;
+    l.shared_tokens = d.has_shared ? tokens : 0;
+    l.experts = d.local_experts; l.list = d.experts; l.hidden = d.hidden; l.ffn = d.ffn; l.gate_bits = d.gate_bits; l.down_bits = d.down_bits;
+    l.split_x = d.act_dtype == ZC_F32 && d.arith != ZC_ARITH_REFERENCE;
+    l.item_split = l.few = tokens * (d.top_k + (d.has_shared ? 1u : 0u)) <= 64;
+    choice[0] = cut.ranks; choice[1] = cut.tokens; choice[3] = 0;
+    choice[2] = !streaming_kernels_fit(l) || item_kernels_pay(l, sms) ? 1 : 2;
     return ZC_OK;
 }
 
@@ -570,12 +577,14 @@ int ep_send_phase(zc_moe* m, uint32_t layer, const void* x, uint32_t tokens, cud
 
 // Owner side: wait for every source's rows, regroup them by expert, run the experts in place, store the results
 // into the senders' windows and publish the return flags.
-int ep_process_phase(zc_moe* m, uint32_t layer, cudaStream_t s) {
+// `tokens`: of each rank (the receive area's capacity says nothing about the load).
+int ep_process_phase(zc_moe* m, uint32_t layer, uint32_t tokens, cudaStream_t s) {
     int n, total = 0;
     Call q = m->ep;
     const LayerMem& L = m->layers[layer];
     q.x = m->ep_window + m->ep_layout.rows; q.records = L.records; q.ids = m->ep_row_ids;
     q.T = m->ep_world * m->ep_layout.cap; q.layer = layer; q.status = m->scratch.status; q.quiet_drop = 1;
+    q.rows_expected = tokens * m->d.top_k;
     if ((n = launch_ep_receive_permute(m, q, s)) < 0) return n;
     if (n == 0) {                           // a receive area too large for one sorting CTA: two launches
         if ((n = launch_ep_receive(m, s)) < 0) return n; total += n;
@@ -604,7 +613,7 @@ int ep_finish_phase(zc_moe* m, uint32_t layer, const void* x, uint32_t tokens, v
 int ep_layer_launches(zc_moe* m, uint32_t layer, const void* x, uint32_t tokens, void* out, cudaStream_t s, void* next) {
     int n, total = 0;
     if ((n = ep_send_phase(m, layer, x, tokens, s)) < 0) return n; total += n;
-    if ((n = ep_process_phase(m, layer, s)) < 0) return n; total += n;
+    if ((n = ep_process_phase(m, layer, tokens, s)) < 0) return n; total += n;
     if ((n = ep_finish_phase(m, layer, x, tokens, out, s, next)) < 0) return n; total += n;
     return total;
 }
@@ -665,7 +674,7 @@ int zc_moe_ep_process(zc_moe* m, uint32_t layer, void* stream) {
     int rc = ep_ready(m, layer);
     if (rc != ZC_OK) return rc;
     DeviceGuard guard(m->device);
-    const int n = ep_process_phase(m, layer, static_cast<cudaStream_t>(stream));
+    const int n = ep_process_phase(m, layer, m->d.max_tokens, static_cast<cudaStream_t>(stream));
     if (n < 0) return n;
     m->launches += n;
     return ZC_OK;

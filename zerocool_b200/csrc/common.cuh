@@ -125,6 +125,7 @@ struct Call {
     uint8_t shared_split;           // the shared record has other bit widths: it runs as launches of its own
     uint8_t act_dtype, out_dtype, meta_f16, router_dtype, has_shared, ref, q8_signed;
     uint32_t item_rows_max;   // decode family: items with more rows than this are left to the tensor-core family (0 = no limit)
+    uint32_t rows_expected;   // routed rows a call can expect where T is a capacity (0: T x K)
     uint8_t quiet_drop;       // the permutation drops ids outside [0, E) without raising the status bit (unused row slots of a receive area)
     // expert parallelism, sender side: the combine waits (bounded) for every owner's return flag of the current epoch
     const unsigned long long* ep_ret_flags;   // [ep_world] in this rank's window; null outside expert parallelism
@@ -290,6 +291,18 @@ RouterCut router_cut(uint32_t tokens, uint32_t experts, bool shared, uint32_t sm
 int launch_route_permute(zc_moe* m, const Call& c, cudaStream_t s, bool do_route, bool do_permute);
 int launch_forced_weights(zc_moe* m, const Call& c, const int32_t* forced, cudaStream_t s);
 int launch_experts_decode(zc_moe* m, const Call& c, cudaStream_t s);
+// What the choice between the decode family's kernels counts (item_kernels_pay in experts_decode.cu).
+struct ExpertLoad {
+    uint32_t rows, shared_tokens;            // routed rows a launch can expect, tokens of the shared expert
+    uint32_t experts, list;                  // experts the rows fall on; entries of the item list
+    uint32_t hidden, ffn, gate_bits, down_bits;
+    bool split_x, split_h;                   // activations / SwiGLU rows as two FP16 terms
+    bool row_limit;                          // the few-row side of a long batch
+    bool item_split;                         // the item kernels would split K over their warps
+    bool few;                                // at most 64 rows and tokens of the shared expert in the layer
+};
+bool item_kernels_pay(const ExpertLoad& l, uint32_t sms);
+bool streaming_kernels_fit(const ExpertLoad& l);
 int launch_experts_item(zc_moe* m, const Call& c, cudaStream_t s);           // one CTA per (item, row tiles): experts_item.cu
 int make_stream_maps(zc_moe* m, LayerMem& L);                                // TMA views of a layer's records (experts_decode.cu)
 int launch_experts_prefill(zc_moe* m, const Call& c, cudaStream_t s, uint32_t skip_rows_upto = 0);

@@ -849,8 +849,9 @@ int launch_experts_decode(zc_moe* m, const Call& c, cudaStream_t s) {
     return total + n;
 }
 
-static bool stream_plan(const zc_moe* m, const Call& c, int nmat, bool split, uint32_t bits, StreamPlan& p) {
-    const uint32_t K = nmat == 2 ? c.H : c.F;
+static bool stream_plan(const ExpertLoad& l, uint32_t sms, int nmat, StreamPlan& p) {
+    const uint32_t K = nmat == 2 ? l.hidden : l.ffn, bits = nmat == 2 ? l.gate_bits : l.down_bits;
+    const bool split = nmat == 2 ? l.split_x : l.split_h;
     p.pairs = (K / 64 + (bits == 4 ? 7 : 3)) / (bits == 4 ? 8 : 4);
     auto fits = [&]() { return stream_smem(p, split, K, bits) <= STREAM_SMEM_MAX; };
     p.warps = MAX_WARPS; p.ks = 1; p.nbuf = 2;
@@ -858,30 +859,57 @@ static bool stream_plan(const zc_moe* m, const Call& c, int nmat, bool split, ui
     // Four warps share a gate/up tile for the shortest batches (one tile per warp would leave most of the SMs without work) and
     // where only one row block fits (hidden above 2560): there the warps of a CTA meet at every pass, and with a quarter of
     // the tiles in flight they arrive closer together (256 tokens at hidden 4096: 492 us against 511 for the layer).
-    if (nmat == 2 && p.pairs >= 4 && (p.nbuf == 1 || c.T * (c.K + (c.has_shared ? 1 : 0)) <= 64)) p.ks = 4;
+    if (nmat == 2 && p.pairs >= 4 && (p.nbuf == 1 || l.few)) p.ks = 4;
     if (!fits()) p.ks = 1;
     while (!fits() && p.warps > 4) p.warps /= 2;
     p.rt = p.warps / p.ks; p.ks_shift = p.ks == 4 ? 2 : 0;
-    p.tiles_per_pass = nmat == 2 ? c.F / 16 : c.H / 32;
-    p.own = (c.E + p.warps * 32 - 1) / (p.warps * 32);
-    p.inv_tiles = 1.0f / float(p.tiles_per_pass); p.inv_grid = 1.0f / float(sm_count(m));
+    p.tiles_per_pass = nmat == 2 ? l.ffn / 16 : l.hidden / 32;
+    p.own = (l.list + p.warps * 32 - 1) / (p.warps * 32);
+    p.inv_tiles = 1.0f / float(p.tiles_per_pass); p.inv_grid = 1.0f / float(sms);
     return fits();
 }
 
-// Batches that stay with the item kernels (csrc/experts_item.cu), whose many small CTAs start faster:
-//  - at most 20 rows: one or two tokens, all latency (1 / 2 tokens of 512 experts: 26.5 / 35.5 us a layer against 30.5 / 37.8);
-//  - where the tiles fill the streaming kernel's warps more than once but less than about twice, so that its second round is
-//    partly empty (12 / 16 tokens: 71.1 / 77.4 us against 72.9 / 81.6; 8 and 20 tokens: 60.4 and 101.5 against 58.4 and 98.5;
-//    hidden 2560, ffn 640: 8 / 12 tokens 76.4 / 96.2 against 82.2 / 97.6, 16 tokens 114 against 117). With hidden 4096 the
-//    item kernels have one CTA per SM and lose from two tokens on. The number of distinct experts is estimated for rows that
-//    fall evenly.
-static bool item_kernels_pay(const zc_moe* m, const Call& c) {
-    const double rows = double(c.T) * c.K, experts = c.local_experts;
-    if (rows <= 20) return true;
-    if (c.H > 2560 || c.item_rows_max) return false;
-    const double passes = experts * (1.0 - std::exp(-rows / experts)) + (c.has_shared ? (c.T + NROW - 1) / NROW : 0);
-    const double rounds = passes * (c.F / 16) / (double(sm_count(m)) * MAX_WARPS);
-    return rounds > 1.2 && rounds < 2.1;
+// Expected number of eight-row passes of `rows` rows that fall evenly on `experts` experts: experts x E[ceil(X / 8)], X Poisson.
+static double expected_passes(double rows, double experts) {
+    if (rows <= 0.0 || experts <= 0.0) return 0.0;
+    const double mean = rows / experts;
+    if (mean > 64.0) return rows / 8.0 + 0.5 * experts;
+    double p = std::exp(-mean), sum = 0.0;
+    for (int x = 1; x < 160; ++x) { p *= mean / x; sum += p * ((x + 7) / 8); }
+    return experts * sum;
+}
+
+// Batches that stay with the item kernels (csrc/experts_item.cu), whose many small CTAs start faster. The figures are item / streaming,
+// us a layer, for loads that fall evenly; `rounds` is how often a launch's gate/up tiles fill the streaming kernel's warps.
+//  - Up to 64 rows and tokens the item kernels split K over eight warps and win while there is little to stream: 0.36 rounds (2 tokens
+//    of 512 experts 35.9 / 37.0, hidden 2560 44.2 / 47.3; 3 tokens of 256 experts 34.3 / 34.1, hidden 2560 45.7 / 46.1), 0.17 rounds with
+//    two-term rows (2 tokens, FP32 activations: streaming 8 - 10 % faster) and above hidden 2560 (hidden 3072: 1 token 37.0 / 39.1, 2 tokens
+//    52.9 / 46.6; hidden 4096: 1 token 44.3 / 45.5 launched one by one though 44.7 / 44.1 from a graph, 2 tokens 61.9 / 52; the shared expert
+//    alone 12.0 / 18.5).
+//  - Beyond, where a round of the streaming kernel is nearly empty and few experts need a second pass: 1.7 to 1.97 rounds (14 / 15 / 16 /
+//    17 tokens 78.2 / 77.2, 78.2 / 78.6, 78.6 / 80.7, 91.5 / 88.9; 14 tokens at ffn 768 of 256 experts 73.3 / 78.8). With a down
+//    projection whose K is not whole stages (ffn 640: ten groups cost twelve) the streaming kernel loses more often: 0.8 to 2.5
+//    rounds, except from 0.47 to 0.82 of a round (512 experts of 2560 / 640: 8 tokens 76.4 / 83.0, 10 tokens 93 / 93, 14 tokens 107.7 /
+//    112.4, 18 tokens 130.2 / 128.8; 64 experts: 24 tokens 70.0 / 72.3, 48 tokens 83.6 / 80.4). Skewed loads (Zipf 1.1) would be better
+//    off streaming there: 16 tokens 72.8 / 54.8, at 2560 / 640 72.2 / 69.8. Above 2.5 rounds even loads gain 1 to 2 % on the item
+//    kernels (22 tokens 145.9 / 149.0) and skewed ones lose 10 (89.4 / 80.9): those batches stream.
+//  - Experts with more rows take further passes, and the codes are dequantised for each: there the streaming kernel
+//    wins (128 experts: 64 tokens 84 / 81, 128 tokens 124 / 114; 512 experts with skewed loads, 64 tokens 302 / 87).
+bool item_kernels_pay(const ExpertLoad& l, uint32_t sms) {
+    const double passes = expected_passes(l.rows, l.experts) + (l.shared_tokens + NROW - 1) / NROW;
+    const double rounds = passes * (l.ffn / 16) / (double(sms) * MAX_WARPS);
+    if (l.row_limit) return false;
+    if (l.item_split) return rounds <= (l.hidden > 2560 || l.split_x ? 0.17 : 0.36);
+    if (l.hidden > 2560 || !l.rows) return false;
+    const double mean = double(l.rows) / l.experts;
+    auto ragged = [](uint32_t K, uint32_t bits) { return (K / 64) % (bits == 4 ? 4 : 2) != 0; };
+    if (!ragged(l.hidden, l.gate_bits) && !ragged(l.ffn, l.down_bits)) return mean <= 1.0 && rounds > 1.7 && rounds < 1.97;
+    const double part = rounds - std::floor(rounds);
+    return mean <= (rounds < 1.2 ? 4.0 : 1.5) && rounds > 0.8 && rounds < 2.5 && !(part > 0.47 && part < 0.82);
+}
+bool streaming_kernels_fit(const ExpertLoad& l) {
+    StreamPlan p{};
+    return stream_plan(l, 148, 2, p) && stream_plan(l, 148, 1, p);
 }
 
 static int launch_experts_decode_one(zc_moe* m, const Call& c, cudaStream_t s) {
@@ -893,10 +921,18 @@ static int launch_experts_decode_one(zc_moe* m, const Call& c, cudaStream_t s) {
     // 2e-3 bound); with the "exact_h" option as two FP16 terms, which costs a second MMA per fragment.
     // The reference arithmetic's h is BF16: exact in one term.
     const bool split_h = !c.ref && m->exact_h;
+    ExpertLoad l{};
+    l.rows = c.items == m->empty_items ? 0 : c.rows_expected ? c.rows_expected : c.T * c.K;
+    l.shared_tokens = c.has_shared ? c.T : 0;
+    l.experts = c.local_experts; l.list = c.E; l.hidden = c.H; l.ffn = c.F; l.gate_bits = c.gate.bits; l.down_bits = c.down.bits;
+    l.split_x = split_x; l.split_h = split_h; l.row_limit = c.item_rows_max != 0;
+    l.item_split = c.T * (c.K + (c.has_shared ? 1 : 0)) <= 64;
+    // The shared expert alone is cut as in its layer's launch, so that its rows are the same bits on every path.
+    l.few = c.rows_expected ? c.rows_expected <= 64 : l.item_split;
     StreamPlan gate_up{}, down{};
-    const bool fits = m->stream_maps && stream_plan(m, c, 2, split_x, c.gate.bits, gate_up) && stream_plan(m, c, 1, split_h, c.down.bits, down);
+    const bool fits = m->stream_maps && stream_plan(l, sm_count(m), 2, gate_up) && stream_plan(l, sm_count(m), 1, down);
     if (m->expert_kernels == 2 && !fits) return fail(m, ZC_EINVAL, "expert_kernels = 2: the streaming kernels do not take this shape");
-    if (m->expert_kernels == 1 || !fits || (m->expert_kernels == 0 && item_kernels_pay(m, c))) return launch_experts_item(m, c, s);
+    if (m->expert_kernels == 1 || !fits || (m->expert_kernels == 0 && item_kernels_pay(l, sm_count(m)))) return launch_experts_item(m, c, s);
     int rc;
     if ((rc = dispatch_expert<2>(m, c, gate_up, split_x, c.gate.bits, m->fold_q4, s)) < 0) return rc;
     if ((rc = dispatch_expert<1>(m, c, down, split_h, c.down.bits, m->fold_q4, s)) < 0) return rc;

@@ -572,9 +572,8 @@ int launch_expert_mb(zc_moe* m, const Call& c, uint32_t items, uint32_t tiles_pe
     if (smem > 220 * 1024) return fail(m, ZC_EINVAL, "expert kernel: shape needs too much shared memory");
     while (tiles_per_warp > 1 && N % (16 * RT * tiles_per_warp)) --tiles_per_warp;
     if (N % (16 * RT * tiles_per_warp)) return fail(m, ZC_EINVAL, "expert kernel: rows not a multiple of the CTA tile");
-    // Items that can have more than eight rows (two or more rows per expert on average, or the few-row side of a long
-    // batch with its limit above eight): their passes run as separate CTAs.
-    const uint32_t pass_ctas = (KS == 1 && (c.item_rows_max > NTOK || uint64_t(c.T) * c.K >= 2ull * c.local_experts)) ? 2u : 1u;
+    // An item can have as many rows as there are tokens: its passes run as separate CTAs (those without a pass leave at once), up to four.
+    const uint32_t pass_ctas = KS == 1 ? (c.T + NTOK - 1) / NTOK < 4 ? (c.T + NTOK - 1) / NTOK : 4u : 1u;
     auto kernel = expert_kernel<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, MBG>;
     static SmemOptIn configured;        // one per instantiation of this function template
     if (opt_in_smem(kernel, configured, m->device, smem) != cudaSuccess) return check_launch(m, "expert kernel attribute");

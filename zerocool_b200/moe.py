@@ -129,13 +129,13 @@ def make_desc(cfg: MoeConfig):
 
 
 def kernel_choice(cfg: MoeConfig, tokens, sms=148):
-    """``zc_moe_kernel_choice``: dict(router_ranks, router_tokens) of a layer call, by the library's rules."""
+    """``zc_moe_kernel_choice``: dict(router_ranks, router_tokens, expert_kernels) of a layer call, by the library's rules."""
     lib = load_library()
     desc, choice = make_desc(cfg), (ctypes.c_uint32 * 4)()
     rc = lib.zc_moe_kernel_choice(ctypes.byref(desc), int(tokens), int(sms), choice)
     if rc != ZC_OK:
         _raise(rc, lib.zc_last_error())
-    return dict(router_ranks=choice[0], router_tokens=choice[1])
+    return dict(router_ranks=choice[0], router_tokens=choice[1], expert_kernels=choice[2])
 
 
 def _raise(code, text):
