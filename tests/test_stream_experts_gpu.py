@@ -168,3 +168,23 @@ def test_received_rows_are_counted_by_tokens_and_not_by_capacity():
     assert all(m.status() == 0 for m in parts)
     assert any(not torch.equal(a, b) for a, b in zip(outs[1], outs[2]))
     assert all(torch.equal(a, b) for a, b in zip(outs[0], outs[2]))
+
+
+@pytest.mark.parametrize("tokens", [5, 40, 1200])
+def test_item_kernels_take_what_the_streaming_kernels_take(tokens):
+    """A handle whose records have no TMA view runs everything on the item kernels, the few-row experts of a long batch too."""
+    torch = pytest.importorskip("torch")
+    from zerocool_b200.moe import Moe
+    cfg = util.cfg2(experts=128, max_tokens=1280)
+    m = Moe(cfg, 0)
+    m.synth_fill_layer(0, SEED)
+    m.set_router_bias(0, synth.zipf_router_bias(cfg, SEED, 0))
+    x = torch.from_numpy(synth.activations(cfg, SEED, 0, tokens)).to(device="cuda", dtype=torch.bfloat16)
+    outs = []
+    for kernels in (2, 1):
+        m.set_option("expert_kernels", kernels)
+        outs.append(m.moe(0, x).clone())
+    counts = np.diff(m.last_routing(tokens)["offsets"])
+    assert tokens < 64 or (((counts > 0) & (counts <= 16)).any() and (counts > 64).any())      # both sides of a long batch
+    assert m.status() == 0
+    assert util.rel_max_error(outs[1].cpu().numpy(), outs[0].cpu().numpy()) <= TOL

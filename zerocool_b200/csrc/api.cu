@@ -224,7 +224,7 @@ int zc_moe_create(const zc_moe_desc* desc, int device, zc_moe** out) {
             A(&L.shared_record, (record_bytes_of(shared_desc_of(d)) + 16383) / 16384 * 16384);
             uint8_t* gw = nullptr; A(&gw, H * elem_bytes(d.router_dtype)); L.shared_gate_w = gw;
         }
-        if (rc == ZC_OK) rc = make_stream_maps(m, L);
+        if (rc == ZC_OK) make_stream_maps(m, L);
     }
     Call& c = m->scratch;
     A(&c.logits, T * E * 4); A(&c.gate_logit, T * 4); A(&c.ids, T * K * 4); A(&c.weights, T * K * 4);

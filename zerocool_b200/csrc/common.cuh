@@ -304,7 +304,7 @@ struct ExpertLoad {
 bool item_kernels_pay(const ExpertLoad& l, uint32_t sms);
 bool streaming_kernels_fit(const ExpertLoad& l);
 int launch_experts_item(zc_moe* m, const Call& c, cudaStream_t s);           // one CTA per (item, row tiles): experts_item.cu
-int make_stream_maps(zc_moe* m, LayerMem& L);                                // TMA views of a layer's records (experts_decode.cu)
+void make_stream_maps(zc_moe* m, LayerMem& L);                               // TMA views of a layer's records (experts_decode.cu)
 int launch_experts_prefill(zc_moe* m, const Call& c, cudaStream_t s, uint32_t skip_rows_upto = 0);
 bool prefill_supported(const zc_moe_desc& d);
 size_t prefill_tile_capacity(const zc_moe_desc& d);

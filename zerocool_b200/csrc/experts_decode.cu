@@ -792,18 +792,19 @@ int dispatch_expert(zc_moe* m, const Call& c, const StreamPlan& p, bool split, u
 }  // namespace
 
 // TMA views of a layer's records (codes of gate and up together: the two projections have one geometry and lie one
-// projection apart; codes of down), encoded once when the handle is created.
-int make_stream_maps(zc_moe* m, LayerMem& L) {
+// projection apart; codes of down), encoded once when the handle is created. Where they cannot be had - a driver without the
+// encoder, or a geometry that it refuses - the handle stays with the item kernels.
+void make_stream_maps(zc_moe* m, LayerMem& L) {
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static Encode encode = nullptr;
-    if (!encode) {
+    static const Encode encode = [] {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q);
-        if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !p) return fail(m, ZC_EEXEC, "cuTensorMapEncodeTiled is not available");
-        encode = reinterpret_cast<Encode>(p);
-    }
+        if (e != cudaSuccess) cudaGetLastError();
+        return reinterpret_cast<Encode>(e == cudaSuccess && q == cudaDriverEntryPointSuccess ? p : nullptr);
+    }();
+    if (!encode) { m->stream_maps = false; return; }
     auto make = [&](StreamMap& to, uint8_t* record, const Projection& pr, uint64_t pair_stride, uint32_t experts, uint64_t stride) {
         const uint64_t row = uint64_t(pr.K) * pr.bits / 8;
         const cuuint64_t dims[4] = {row, pr.N, pair_stride ? 2u : 1u, experts};
@@ -824,8 +825,7 @@ int make_stream_maps(zc_moe* m, LayerMem& L) {
         const uint64_t stride = (record_bytes_of(sd) + 16383) / 16384 * 16384;
         ok = make(L.map_shared_gate_up, L.shared_record, sg, su.codes - sg.codes, 1, stride) && make(L.map_shared_down, L.shared_record, sdn, 0, 1, stride);
     }
-    m->stream_maps = m->stream_maps && ok;      // a geometry TMA cannot describe stays with the item kernels
-    return ZC_OK;
+    m->stream_maps = m->stream_maps && ok;
 }
 
 static int launch_experts_decode_one(zc_moe* m, const Call& c, cudaStream_t s);
