@@ -40,7 +40,7 @@
 // Activations must stay inside FP16 after the factor 16 (|x| < 4094 for Q4 projections, < 65504 for Q8); hidden
 // states after a norm are O(1..100). A value beyond that raises ZC_STATUS_RANGE in the status word (the output of
 // that row is then not meaningful); the same holds for the SwiGLU rows the down projection reads.
-#include "common.cuh"
+#include "experts_common.cuh"
 
 namespace zc {
 namespace {
@@ -48,7 +48,6 @@ namespace {
 constexpr int NTOK = 8;               // token rows per MMA pass (the N of m16n8k16)
 constexpr int WARPS = 8;
 constexpr int EXPERT_THREADS = WARPS * 32;
-constexpr int ROW_PAD = 8;            // halves added to each staged row (keeps 16-byte reads conflict free)
 #ifndef ZC_MIN_BLOCKS
 #define ZC_MIN_BLOCKS 2
 #endif
@@ -75,27 +74,8 @@ template <int BITS, int CHT> struct Fmt {
     __host__ __device__ static constexpr uint32_t swizzle(uint32_t row) { return (row / ROWS_PER_WINDOW) & (CHT - 1); }
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// D(16x8, fp32) += A(16x16, fp16, row) * B(16x8, fp16, col). Lane (g = lane/4, c = lane%4) holds
-//   a0: A[g][2c,2c+1]   a1: A[g+8][2c,2c+1]   a2: A[g][2c+8,2c+9]   a3: A[g+8][2c+8,2c+9]
-//   b0: B[2c,2c+1][g]   b1: B[2c+8,2c+9][g]
-//   d0,d1: D[g][2c,2c+1]   d2,d3: D[g+8][2c,2c+1]
-__device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// Same product with the addend taken from c (the first MMA of a group starts from the folded offset).
-__device__ __forceinline__ void mma_f16_16816_c(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
-                                                float c0, float c1, float c2, float c3) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
-}
 
 // Ring depth per warp: two stages of four groups or three of two keep the same bytes in flight.
 __host__ __device__ constexpr int stages_for(int matrices_per_warp, int ch) { return (ch == 4 && matrices_per_warp == 2) ? 2 : 3; }
@@ -132,18 +112,15 @@ __device__ __forceinline__ bool decode_item(const Call& c, uint32_t item, ItemIn
     return true;
 }
 
-// Stage the valid source rows (n < nvalid) of K elements into shared memory as FP16 (hi, and lo when
-// SPLIT), in the k order the MMA fragments expect, with the per-group sums
-//   sums[grp][n] = (Sx, P):  Sx = sum of x over the group (REF: the reference's BF16 sum of four,
-//   qwen.metal:55), P = -1024 * sum of the values as staged: the MMA accumulator starts from P, which
-//   removes the folded 1024 offset of the codes (0 without FOLD).
-//   Q4 order inside each block of 8: (0,4,1,5,2,6,3,7), even k staged x 16 when FOLD; Q8: natural order.
+// Stage the valid source rows (n < nvalid) of K elements into shared memory (convert8: hi, lo, and per group)
+//   sums[grp][n] = (sx, P), P = -1024 * sf: the MMA accumulator starts from P, which removes the folded 1024 offset of the codes
+//   (0 without FOLD).
 // Rows n >= nvalid are left as they are: an MMA column only depends on its own B column.
 template <bool Q4ORDER, bool SPLIT, bool FOLD>
 __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, const int* rows, uint32_t nvalid,
                                            uint32_t K, bool ref, __half* hi, __half* lo, float* sums, uint32_t* status) {
     const uint32_t RS = K + ROW_PAD, blocks = K / 8, total = nvalid * blocks;
-    bool out_of_range = false;
+    float most = 0.0f;
     // The trip count is uniform per warp (the shuffles below need all 32 lanes); lanes past the end carry zeros.
     for (uint32_t idx = threadIdx.x; (idx & ~31u) < total; idx += EXPERT_THREADS) {
         const bool live = idx < total;
@@ -163,47 +140,15 @@ __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, const 
 #pragma unroll
             for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(r[i] << 16); v[2 * i + 1] = __uint_as_float(r[i] & 0xffff0000u); }
         }
-        float sx;
-        if (ref) sx = bf_round(bf_round(bf_round(v[0] + v[1]) + v[2]) + v[3]) + bf_round(bf_round(bf_round(v[4] + v[5]) + v[6]) + v[7]);
-        else sx = (((v[0] + v[1]) + v[2]) + v[3]) + (((v[4] + v[5]) + v[6]) + v[7]);
-        __half h[8], l[8];
-        float sf = 0.0f, sn = 0.0f;        // sums of the values as fed to the MMA: as staged, and in natural scale
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            // folded Q4 codes: the value that meets a "1024 + 16 q" slot must be 1/16 of its neighbours'. Even slots are
-            // staged x 16 rather than odd slots / 16, which keeps small activations out of FP16's subnormal range; the
-            // accumulated result is multiplied by 1/16 (exact) when it is finished.
-            const float pre = (FOLD && Q4ORDER && !(i & 1)) ? v[i] * 16.0f : v[i];
-            out_of_range |= fabsf(pre) > 65504.0f;          // would become an FP16 infinity: reported, not hidden
-            h[i] = __float2half_rn(pre);
-            float fed = __half2float(h[i]);
-            if (SPLIT) { l[i] = __float2half_rn(pre - fed); fed += __half2float(l[i]); }
-            sf += fed;
-            sn += (FOLD && Q4ORDER && !(i & 1)) ? fed * 0.0625f : fed;
-        }
-        // The bias term multiplies the sum of the activations. Outside the reference arithmetic it uses the sum of
-        // the values the MMA really sees, so that a rounding of an activation to FP16 enters the result through the
-        // weight s q + b and not through s q alone.
-        if (!ref) sx = sn;
-#pragma unroll
-        for (int off = 1; off <= 4; off <<= 1) {
-            sx += __shfl_xor_sync(0xffffffffu, sx, off);
-            sf += __shfl_xor_sync(0xffffffffu, sf, off);
-        }
+        uint4 ph, pl;
+        float sx, sf;
+        convert8<Q4ORDER, SPLIT, FOLD>(v, ref, ph, pl, sx, sf, most);
         if (!live) continue;
-        if ((q & 7) == 0) *reinterpret_cast<float2*>(sums + ((q / 8) * NTOK + n) * 2) = make_float2((FOLD && Q4ORDER) ? 16.0f * sx : sx, FOLD ? -1024.0f * sf : 0.0f);
-        constexpr int order_q4[8] = {0, 4, 1, 5, 2, 6, 3, 7};
-        uint32_t ph[4], pl[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int a = Q4ORDER ? order_q4[2 * i] : 2 * i, b = Q4ORDER ? order_q4[2 * i + 1] : 2 * i + 1;
-            ph[i] = uint32_t(__half_as_ushort(h[a])) | (uint32_t(__half_as_ushort(h[b])) << 16);
-            if (SPLIT) pl[i] = uint32_t(__half_as_ushort(l[a])) | (uint32_t(__half_as_ushort(l[b])) << 16);
-        }
-        *reinterpret_cast<uint4*>(hi + n * RS + q * 8) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-        if (SPLIT) *reinterpret_cast<uint4*>(lo + n * RS + q * 8) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+        if ((q & 7) == 0) *reinterpret_cast<float2*>(sums + ((q / 8) * NTOK + n) * 2) = make_float2(sx, FOLD ? -1024.0f * sf : 0.0f);
+        *reinterpret_cast<uint4*>(hi + n * RS + q * 8) = ph;
+        if (SPLIT) *reinterpret_cast<uint4*>(lo + n * RS + q * 8) = pl;
     }
-    if (out_of_range) atomicOr(status, ZC_STATUS_RANGE);
+    if (!(most <= 65504.0f)) atomicOr(status, ZC_STATUS_RANGE);        // would become an FP16 infinity: reported, not hidden
 }
 
 // Source of one matrix for this lane's cp.async copies. A pass of the warp copies ROWS_PER_PASS rows: the
@@ -254,44 +199,6 @@ __device__ __forceinline__ void issue_matrix(uint32_t stage, uint32_t meta_area,
     } else {
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(meta_area + meta_buf * (32 * CHT * 2) + src.meta_pair * CHT * 2), "l"(src.tile_meta + grp0 * 2) : "memory");
     }
-}
-
-// (a & b) | c in one logic instruction.
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
-// Q4: one word -> four half2 (k0,k4) (k1,k5) (k2,k6) (k3,k7) of its 8 codes.
-template <bool FOLD>
-__device__ __forceinline__ void dequant_q4(uint32_t w, uint32_t (&p)[4]) {
-    const uint32_t lo = 0x000f000fu, hi = 0x00f000f0u, magic = 0x64006400u;
-    const uint32_t w8 = w >> 8;
-    p[0] = and_or(w, lo, magic);
-    p[1] = and_or(w, hi, magic);
-    p[2] = and_or(w8, lo, magic);
-    p[3] = and_or(w8, hi, magic);
-    if (!FOLD) {
-        const __half2 k1024 = __floats2half2_rn(1024.0f, 1024.0f), k16 = __floats2half2_rn(0.0625f, 0.0625f), k64 = __floats2half2_rn(-64.0f, -64.0f);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            __half2 v = *reinterpret_cast<__half2*>(&p[i]);
-            v = (i & 1) ? __hfma2(v, k16, k64) : __hsub2(v, k1024);
-            p[i] = *reinterpret_cast<uint32_t*>(&v);
-        }
-    }
-}
-// Q8: one word -> two half2 (k0,k1) (k2,k3); every integer in [-128, 255] is exact in FP16.
-__device__ __forceinline__ void dequant_q8(uint32_t w, bool is_signed, uint32_t (&p)[2]) {
-    if (is_signed) w ^= 0x80808080u;
-    const float off = is_signed ? 8388608.0f + 128.0f : 8388608.0f;
-    float f[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) f[i] = __uint_as_float(0x4b000000u | ((w >> (8 * i)) & 0xffu)) - off;
-    const __half2 a = __floats2half2_rn(f[0], f[1]), b = __floats2half2_rn(f[2], f[3]);
-    p[0] = *reinterpret_cast<const uint32_t*>(&a);
-    p[1] = *reinterpret_cast<const uint32_t*>(&b);
 }
 
 // d(16 rows x 8 tokens) = sum over one 64-wide group of code * x for the lane's rows g (w0) and g+8 (w1).
