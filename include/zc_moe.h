@@ -298,12 +298,7 @@ int zc_moe_stack_host(zc_moe* moe, const void* x_host, uint32_t tokens, void* ou
  *   kernels and the grouped GEMM takes the others (0: the grouped GEMM takes every expert).
  *   "expert_kernels" (default 0): which kernels run the decode family's experts: 0 by the batch, 1 the item kernels, 2 the
  *   streaming kernels (ZC_EINVAL from a call whose shape they do not take). The two differ in the order of FP32 sums.
- *   "few_tiles_gate_up" (default 1), "few_tiles_down" (default 2), 1..4: 16-row tiles per warp of the item kernels in such
- *   launches; "meta_blocks" (default 1): the item kernels fetch scales and biases eight groups at a time (16-byte copies)
- *   for gate/up at hidden >= 4096; 2 does so wherever the layout allows, 3 uses four-group blocks for gate/up, 0 never
- *   (each ring stage's own halves, 4- or 8-byte copies). Both matter only where a batch runs on the item kernels (one or two
- *   tokens, and some short batches: csrc/experts_decode.cu has the rule). Results are identical.
- *   "router_db" (0 or 1): accepted, without effect (long batches have one router form). Results are identical.
+ *   "few_tiles_gate_up", "few_tiles_down" (1..4), "meta_blocks" (0..3), "router_db" (0, 1): accepted, without effect.
  * Changing an option drops the cached graphs of zc_moe_stack. */
 int zc_moe_set_option(zc_moe* moe, const char* name, int value);
 

@@ -12,6 +12,7 @@ from oracle import oracle
 from tests import util
 from tests.test_moe_gpu import TOL, device_x, make, oracle_layer
 from zerocool_b200 import synth
+from zerocool_b200.moe import kernel_choice
 from zerocool_b200.records import ARITH_REFERENCE, BF16, F32, MoeConfig
 
 pytestmark = pytest.mark.gpu
@@ -487,44 +488,49 @@ def test_few_row_experts_take_the_streaming_kernels_in_a_long_batch():
         m.set_option("prefill_small_rows", 65)
 
 
+@pytest.mark.parametrize("kernels", [1, 2])
 @pytest.mark.parametrize("tokens", [5, 40])
-def test_metadata_blocks_give_the_same_bits(tokens):
-    """hidden 4096 (config 5's geometry): scales and biases fetched eight groups at a time (default) or per ring stage
-    (option meta_blocks = 0) feed the same arithmetic: identical bits, and within tolerance of the CPU checker."""
+def test_both_expert_kernels_at_hidden_4096(tokens, kernels):
+    """hidden 4096 (config 5's geometry) on the item and on the streaming kernels: within tolerance of the CPU checker, and the
+    accepted option meta_blocks changes nothing."""
     import torch
     cfg = util.cfg2(hidden=4096, experts=32, top_k=4, max_tokens=64)
     m = make(cfg)
     m.synth_fill_layer(0, SEED)
+    m.set_option("expert_kernels", kernels)
     x = synth.activations(cfg, SEED, 0, tokens)
-    blocks = m.decode(0, device_x(m, x)).clone()
+    out = m.decode(0, device_x(m, x)).clone()
     m.set_option("meta_blocks", 0)
-    stages = m.decode(0, device_x(m, x)).clone()
+    assert torch.equal(m.decode(0, device_x(m, x)), out)
     assert m.status() == 0
-    assert torch.equal(blocks, stages)
     routing = m.last_routing(tokens)
     records = util.selected_records(cfg, SEED, 0, routing["ids"])
     want = oracle.moe_layer(cfg.as_dict(), records, synth.router(cfg, SEED, 0), x,
                             shared_record=synth.record(cfg, SEED, 0, synth.SHARED_EXPERT), shared_gate_w=synth.shared_gate(cfg, SEED, 0))
     assert np.array_equal(routing["ids"], want["ids"])
-    assert util.rel_max_error(blocks.float().cpu().numpy(), want["out"]) <= TOL
+    assert util.rel_max_error(out.float().cpu().numpy(), want["out"]) <= TOL
 
 
 def test_tuning_switches_do_not_change_a_bit():
-    """Every switch that only moves work around (copy sizes of the metadata, CTAs per few-row expert, router tile
-    buffering, prefetch form, dependent launches) must leave a long batch and a short batch bit-identical."""
+    """Dependent launches on or off leave a long batch and short batches on either family of expert kernels bit-identical, and
+    so do the options that are accepted without effect."""
     import torch
     cfg = util.cfg2(max_tokens=1280)
+    assert [kernel_choice(cfg, t)["expert_kernels"] for t in (24, 16)] == [2, 1]
     m = make(cfg)
     m.synth_fill_layer(0, SEED)
     m.set_router_bias(0, synth.zipf_router_bias(cfg, SEED, 0))
     long_x = device_x(m, synth.activations(cfg, SEED, 0, 1200))          # whole-K router tiles, hybrid dispatch, many-CTA permutation
-    short_x = device_x(m, synth.activations(cfg, SEED, 1, 24))
-    base_long, base_short = m.moe(0, long_x).clone(), m.moe(0, short_x).clone()
+    short_x = device_x(m, synth.activations(cfg, SEED, 1, 24))           # streaming kernels
+    item_x = device_x(m, synth.activations(cfg, SEED, 1, 16))            # item kernels
+    base_long, base_short, base_item = m.moe(0, long_x).clone(), m.moe(0, short_x).clone(), m.moe(0, item_x).clone()
+    m.moe(0, short_x)
     ids_long = m.last_routing(24)["ids"].copy()
     for name, value, restore in (("meta_blocks", 0, 1), ("meta_blocks", 2, 1), ("meta_blocks", 3, 1), ("few_tiles_gate_up", 2, 1),
                                  ("few_tiles_down", 4, 2), ("router_db", 0, 1), ("pdl", 0, 1)):
         m.set_option(name, value)
         assert torch.equal(m.moe(0, long_x), base_long), (name, value)
+        assert torch.equal(m.moe(0, item_x), base_item), (name, value)
         assert torch.equal(m.moe(0, short_x), base_short), (name, value)
         assert np.array_equal(m.last_routing(24)["ids"], ids_long)
         m.set_option(name, restore)

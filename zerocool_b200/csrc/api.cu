@@ -925,24 +925,12 @@ int zc_moe_set_option(zc_moe* m, const char* name, int value) {
         m->expert_kernels = uint32_t(value);
         return ZC_OK;
     }
-    if (!std::strcmp(name, "few_tiles_gate_up") || !std::strcmp(name, "few_tiles_down")) {
-        if (value < 1 || value > 4) return fail(m, ZC_EINVAL, "few_tiles_* must be 1..4");
-        DeviceGuard guard(m->device);
-        drop_graphs(m);
-        (name[10] == 'g' ? m->few_tiles_gate_up : m->few_tiles_down) = uint32_t(value);
-        return ZC_OK;
-    }
-    if (!std::strcmp(name, "router_db")) {
-        if (value != 0 && value != 1) return fail(m, ZC_EINVAL, "router_db must be 0 or 1");
-        return ZC_OK;                        // both forms it chose between are one kernel now
-    }
-    if (!std::strcmp(name, "meta_blocks")) {
-        if (value < 0 || value > 3) return fail(m, ZC_EINVAL, "meta_blocks must be 0..3");
-        DeviceGuard guard(m->device);
-        drop_graphs(m);
-        m->meta_blocks = uint32_t(value);
-        return ZC_OK;
-    }
+    // Choices that earlier kernels had: still accepted.
+    const struct { const char* name; int low, high; const char* error; } retired[] = {
+        {"few_tiles_gate_up", 1, 4, "few_tiles_* must be 1..4"}, {"few_tiles_down", 1, 4, "few_tiles_* must be 1..4"},
+        {"meta_blocks", 0, 3, "meta_blocks must be 0..3"}, {"router_db", 0, 1, "router_db must be 0 or 1"}};
+    for (const auto& r : retired)
+        if (!std::strcmp(name, r.name)) return value < r.low || value > r.high ? fail(m, ZC_EINVAL, r.error) : ZC_OK;
     if (!std::strcmp(name, "ep_wait_ms")) {
         if (value < 1 || value > 60000) return fail(m, ZC_EINVAL, "ep_wait_ms must be 1..60000");
         DeviceGuard guard(m->device);

@@ -65,9 +65,8 @@ template <int BITS, int CHT> struct Fmt {
     static constexpr int PASSES = 16 / ROWS_PER_PASS;
     static constexpr int CODES = 16 * LINE;
     static constexpr int MATRIX = CODES;                  // a ring stage holds the codes only
-    // Metadata of a matrix, beside the ring: [buffer][row][scale, bias][MG halves]. MG = 8 groups per block (one 16-byte
-    // copy per (row, kind), two buffers) where a warp walks K in order, else MG = CHT (one block per ring stage).
-    __host__ __device__ static constexpr int meta_area(int mbg, int stages) { return mbg ? 2 * 32 * mbg * 2 : stages * 32 * CHT * 2; }     // bytes per matrix per warp (mbg: groups per block, 0 = per stage)
+    // Metadata of a matrix, beside the ring: [ring stage][row][scale, bias][CHT halves].
+    __host__ __device__ static constexpr int meta_area(int stages) { return stages * 32 * CHT * 2; }     // bytes per matrix per warp
     // Rows whose lines fall into the same 128-byte bank window are ROWS_PER_WINDOW apart; the block index of a row is
     // xor-ed with swizzle(row) so that rows read together by one MMA fragment load use different banks.
     static constexpr int ROWS_PER_WINDOW = LINE >= 128 ? 1 : 128 / LINE;
@@ -178,27 +177,19 @@ struct LaneSource {
     }
 };
 
-// Issue the cp.async copies of one chunk (CHT groups starting at grp0) of one matrix into a ring stage, and the
-// metadata that goes with it. MB8: one 16-byte copy per (row, kind) every eight groups, into buffer meta_buf of two (a
-// 4-byte copy per chunk moves a whole 32-byte sector for it and costs as many shared-memory wavefronts as a code copy);
-// otherwise the chunk's own scale and bias halves, into the buffer of its ring slot.
-template <int BITS, int CHT, int MBG>
-__device__ __forceinline__ void issue_matrix(uint32_t stage, uint32_t meta_area, const LaneSource<BITS, CHT>& src, uint32_t grp0, uint32_t meta_buf, bool meta_now) {
+// Issue the cp.async copies of one chunk (CHT groups starting at grp0) of one matrix into a ring stage, and its scale and bias
+// halves into the stage's place in the metadata area.
+template <int BITS, int CHT>
+__device__ __forceinline__ void issue_matrix(uint32_t stage, uint32_t meta_area, const LaneSource<BITS, CHT>& src, uint32_t grp0, uint32_t slot) {
     using F = Fmt<BITS, CHT>;
     const uint8_t* g0 = src.tile_codes + grp0 * F::ROWB;
 #pragma unroll
     for (int p = 0; p < F::PASSES; ++p)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(stage + src.dst0 + p * F::ROWS_PER_PASS * F::LINE),
                      "l"(g0 + size_t(p * F::ROWS_PER_PASS) * src.row_bytes) : "memory");
-    if constexpr (MBG == 8) {
-        if (meta_now) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(meta_area + meta_buf * 512 + src.meta_pair * 16), "l"(src.tile_meta + grp0 * 2) : "memory");
-    } else if constexpr (MBG == 4) {
-        if (meta_now) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(meta_area + meta_buf * 256 + src.meta_pair * 8), "l"(src.tile_meta + grp0 * 2) : "memory");
-    } else if constexpr (CHT == 4) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(meta_area + meta_buf * (32 * CHT * 2) + src.meta_pair * CHT * 2), "l"(src.tile_meta + grp0 * 2) : "memory");
-    } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(meta_area + meta_buf * (32 * CHT * 2) + src.meta_pair * CHT * 2), "l"(src.tile_meta + grp0 * 2) : "memory");
-    }
+    const uint32_t to = meta_area + slot * (32 * CHT * 2) + src.meta_pair * CHT * 2;
+    if constexpr (CHT == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(src.tile_meta + grp0 * 2) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(src.tile_meta + grp0 * 2) : "memory");
 }
 
 // d(16 rows x 8 tokens) = sum over one 64-wide group of code * x for the lane's rows g (w0) and g+8 (w1).
@@ -246,17 +237,14 @@ __device__ __forceinline__ void group_mma(float (&d)[4], float c0, float c1, con
 //       go to two different warps, which halves the registers and ring of a warp (three CTAs per SM instead
 //       of two) at the price of meeting in shared memory for the SwiGLU.
 //   CH: quantisation groups per ring stage (4 when K is a multiple of 256, else 2; Q8 always 2).
-//   MBG: scales and biases arrive MBG = 8 or 4 groups at a time (needs KS = 1 and a group count that is a multiple of MBG); 0: with every ring stage.
-template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH, int MBG>
+template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH>
 __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN : (MW == 2 ? 3 : ZC_MIN_BLOCKS)) expert_kernel(Call c, uint32_t tiles_per_warp) {
     using F = Fmt<BITS, CH>;
     constexpr int STAGES = stages_for(NMAT / MW, CH);
     constexpr int WM = NMAT / MW;                    // matrices per warp
     constexpr int RT = WARPS / (KS * MW);
     constexpr int STAGE = WM * F::MATRIX;
-    constexpr int META_AREA = F::meta_area(MBG, STAGES);
-    constexpr bool MB8 = MBG != 0;                   // metadata in blocks of MBG groups
-    constexpr int MBLOCK = MBG ? MBG : 8;
+    constexpr int META_AREA = F::meta_area(STAGES);
     constexpr bool VIA_SMEM = KS > 1 || MW > 1;
     constexpr int WORDS = F::ROWB / 16;              // 32-bit words per lane per row per group: 2 (Q4) / 4 (Q8)
     constexpr bool FOLDQ = FOLD && BITS == 4;
@@ -299,18 +287,14 @@ __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN
     for (uint32_t pass = blockIdx.z; pass * NTOK < it.count; pass += gridDim.z) {
         const uint32_t nvalid = min(uint32_t(NTOK), it.count - pass * NTOK);
         uint32_t is_tile = 0, is_chunk = 0, is_slot = 0;        // producer position in the flattened (tile, chunk) sequence
-        uint32_t is_mblk = 0;                  // MB8: metadata blocks issued so far; the next one goes to buffer is_mblk & 1
         const uint32_t ring_base = smem_u32(my_ring), meta_base = smem_u32(my_meta);
 #pragma unroll
         for (int m = 0; m < WM; ++m) src[m].set_tile(first_tile * 16, G);
         auto issue = [&]() {
             if (is_tile < my_tiles) {
                 const uint32_t stage = ring_base + is_slot * STAGE, grp0 = (ks + is_chunk * KS) * CH;
-                const bool meta_now = MB8 && (is_chunk * CH) % MBLOCK == 0;
-                const uint32_t meta_buf = MB8 ? (is_mblk & 1) : is_slot;
 #pragma unroll
-                for (int m = 0; m < WM; ++m) issue_matrix<BITS, CH, MBG>(stage + m * F::MATRIX, meta_base + m * META_AREA, src[m], grp0, meta_buf, meta_now);
-                if (meta_now) ++is_mblk;
+                for (int m = 0; m < WM; ++m) issue_matrix<BITS, CH>(stage + m * F::MATRIX, meta_base + m * META_AREA, src[m], grp0, is_slot);
                 if (++is_chunk == my_n) {
                     is_chunk = 0; ++is_tile;
 #pragma unroll
@@ -357,7 +341,7 @@ __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN
             }
         };
 
-        uint32_t slot = 0, mblk = 0;           // mblk: metadata blocks the consumer has begun (MB8)
+        uint32_t slot = 0;
         for (uint32_t tile = 0; tile < tiles_per_warp; ++tile) {
             float acc[WM][4];
 #pragma unroll
@@ -366,10 +350,7 @@ __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN
                 cp_async_wait<STAGES - 2>();
                 __syncwarp();
                 const uint8_t* stage = my_ring + slot * STAGE;
-                // this chunk's scale and bias halves: at its place in the current 8-group block (MB8), or in the buffer of its slot
-                if (MB8 && (i * CH) % MBLOCK == 0) ++mblk;
-                constexpr uint32_t PAIR = MB8 ? uint32_t(MBLOCK * 2) : uint32_t(CH * 2);          // bytes of one (row, kind) entry
-                const uint8_t* mbase = MB8 ? my_meta + ((mblk - 1) & 1) * (32 * PAIR) + ((i * CH) % MBLOCK) * 2 : my_meta + slot * (32 * CH * 2);
+                const uint8_t* mbase = my_meta + slot * (32 * CH * 2);                            // this chunk's scale and bias halves
                 slot = slot + 1 == STAGES ? 0 : slot + 1;
                 issue();          // refills the slot consumed by the previous iteration while this chunk is multiplied
                 const uint32_t grp0 = (ks + i * KS) * CH;
@@ -378,12 +359,10 @@ __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN
                 for (int m = 0; m < WM; ++m) {
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
-                        const uint8_t* mp = mbase + m * META_AREA + (g + 8 * r) * 2 * PAIR;
+                        const uint8_t* mp = mbase + m * META_AREA + (g + 8 * r) * 4 * CH;
                         if constexpr (CH == 4) {
-                            const uint2 sc = *reinterpret_cast<const uint2*>(mp), bi = *reinterpret_cast<const uint2*>(mp + PAIR);
+                            const uint2 sc = *reinterpret_cast<const uint2*>(mp), bi = *reinterpret_cast<const uint2*>(mp + 2 * CH);
                             mraw[m][r][0] = sc.x; mraw[m][r][1] = sc.y; mraw[m][r][2] = bi.x; mraw[m][r][3] = bi.y;
-                        } else if constexpr (MB8) {
-                            mraw[m][r][0] = *reinterpret_cast<const uint32_t*>(mp); mraw[m][r][1] = *reinterpret_cast<const uint32_t*>(mp + PAIR);
                         } else {
                             const uint2 v = *reinterpret_cast<const uint2*>(mp);
                             mraw[m][r][0] = v.x; mraw[m][r][1] = v.y;
@@ -469,45 +448,25 @@ __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN
     }
 }
 
-template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH, int MBG>
-int launch_expert_mb(zc_moe* m, const Call& c, uint32_t items, uint32_t tiles_per_warp, cudaStream_t s) {
+template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH>
+int launch_expert_ch(zc_moe* m, const Call& c, uint32_t items, uint32_t tiles_per_warp, cudaStream_t s) {
     constexpr int RT = WARPS / (KS * MW);
     constexpr int STAGES = stages_for(NMAT / MW, CH);
     const uint32_t K = NMAT == 2 ? c.H : c.F, N = NMAT == 2 ? c.F : c.H, G = K / 64;
     const size_t smem = size_t(SPLIT ? 2 : 1) * NTOK * (K + ROW_PAD) * 2 + size_t(G) * NTOK * 2 * 4 +
-                        size_t(WARPS) * (NMAT / MW) * (STAGES * Fmt<BITS, CH>::MATRIX + Fmt<BITS, CH>::meta_area(MBG, STAGES)) + ((KS > 1 || MW > 1) ? size_t(KS) * NMAT * RT * 16 * NTOK * 4 : 0);
+                        size_t(WARPS) * (NMAT / MW) * (STAGES * Fmt<BITS, CH>::MATRIX + Fmt<BITS, CH>::meta_area(STAGES)) + ((KS > 1 || MW > 1) ? size_t(KS) * NMAT * RT * 16 * NTOK * 4 : 0);
     if (smem > 220 * 1024) return fail(m, ZC_EINVAL, "expert kernel: shape needs too much shared memory");
     while (tiles_per_warp > 1 && N % (16 * RT * tiles_per_warp)) --tiles_per_warp;
     if (N % (16 * RT * tiles_per_warp)) return fail(m, ZC_EINVAL, "expert kernel: rows not a multiple of the CTA tile");
     // An item can have as many rows as there are tokens: its passes run as separate CTAs (those without a pass leave at once), up to four.
     const uint32_t pass_ctas = KS == 1 ? (c.T + NTOK - 1) / NTOK < 4 ? (c.T + NTOK - 1) / NTOK : 4u : 1u;
-    auto kernel = expert_kernel<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, MBG>;
+    auto kernel = expert_kernel<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH>;
     static SmemOptIn configured;        // one per instantiation of this function template
     if (opt_in_smem(kernel, configured, m->device, smem) != cudaSuccess) return check_launch(m, "expert kernel attribute");
     Timed t(m, s, NMAT == 2 ? KERNEL_GATE_UP : KERNEL_DOWN);
     const cudaError_t e = launch_chained(m, NMAT == 2 ? KERNEL_GATE_UP : KERNEL_DOWN, kernel, dim3(N / (16 * RT * tiles_per_warp), items, pass_ctas), dim3(EXPERT_THREADS), smem, s, nullptr, 0, c, tiles_per_warp);
     if (e != cudaSuccess) return fail(m, ZC_EEXEC, std::string("expert kernel launch: ") + cudaGetErrorString(e));
     return check_launch(m, NMAT == 2 ? "gate_up" : "down");
-}
-
-// Metadata in 8-group blocks: possible where a warp walks K in order (KS = 1) and every block of a row's metadata is
-// 16-byte aligned; used for gate/up with long rows (hidden 4096: 423 -> 368 us at 512 experts x 5 rows). With short rows
-// the extra kilobyte per warp pushes two CTAs per SM over a shared-memory carve-out step, which costs the L1 that serves
-// the small copies (97 -> 104 us at hidden 2048), and down's short K does not gain (56 -> 58 us): those keep one block per
-// ring stage. Option meta_blocks: 0 never, 1 by this rule, 2 wherever possible, 3 four-group blocks for gate/up.
-template <int BITS, bool SPLIT, int NMAT, int KS, bool FOLD, bool META_F16, int MW, int CH>
-int launch_expert_ch(zc_moe* m, const Call& c, uint32_t items, uint32_t tiles_per_warp, cudaStream_t s) {
-    if constexpr (KS == 1) {
-        const uint32_t K = NMAT == 2 ? c.H : c.F, G = K / 64;
-        const bool long_rows = NMAT == 2 && K >= 4096;
-        if (G % 8 == 0 && (m->meta_blocks == 2 || (m->meta_blocks == 1 && long_rows)))
-            return launch_expert_mb<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, 8>(m, c, items, tiles_per_warp, s);
-        if constexpr (CH == 2 && NMAT == 2) {       // 4-group blocks (8-byte copies every second stage; stays inside the carve-out): 99.7 against 98.1 us at hidden 2048, so only on request
-            if (G % 4 == 0 && m->meta_blocks == 3)
-                return launch_expert_mb<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, 4>(m, c, items, tiles_per_warp, s);
-        }
-    }
-    return launch_expert_mb<BITS, SPLIT, NMAT, KS, FOLD, META_F16, MW, CH, 0>(m, c, items, tiles_per_warp, s);
 }
 
 // Two groups per ring stage for gate/up: four groups per stage (a full 128-byte line per Q4 row) leave room for
@@ -554,18 +513,10 @@ int launch_experts_item(zc_moe* m, const Call& c, cudaStream_t s) {
     const bool small = c.T * (c.K + (c.has_shared ? 1 : 0)) <= 64;
     int rc;
     if (small) rc = dispatch_expert<2, 8>(m, c, items, 1, split_x, c.gate.bits, fold, s);
-#ifndef ZC_TPW_GU
-#define ZC_TPW_GU 2
-#endif
-#ifndef ZC_TPW_DN
-#define ZC_TPW_DN 4
-#endif
-    // As the few-row side of a long batch only a fraction of the items has work (the others leave at once): fewer
-    // tiles per warp, i.e. more and shorter CTAs per item, keep the SMs filled.
-    else rc = dispatch_expert<2, 1>(m, c, items, c.item_rows_max ? m->few_tiles_gate_up : ZC_TPW_GU, split_x, c.gate.bits, fold, s);
+    else rc = dispatch_expert<2, 1>(m, c, items, 2, split_x, c.gate.bits, fold, s);
     if (rc < 0) return rc;
     if (small) rc = dispatch_expert<1, 2>(m, c, items, 1, split_h, c.down.bits, fold, s);
-    else rc = dispatch_expert<1, 1>(m, c, items, c.item_rows_max ? m->few_tiles_down : ZC_TPW_DN, split_h, c.down.bits, fold, s);
+    else rc = dispatch_expert<1, 1>(m, c, items, 4, split_h, c.down.bits, fold, s);
     if (rc < 0) return rc;
     return 2;
 }
