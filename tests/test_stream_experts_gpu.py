@@ -1,6 +1,7 @@
 """The persistent streaming expert kernels against the CPU checker, at the sizes where their cut can go wrong: K that is not
 whole stages or pairs of stages, one staged row block, warps sharing a tile, more passes per CTA than its table holds, long
-items, FP32 activations, 8-bit codes, and biases that do not follow the scales (the bias product on its own)."""
+items, more list entries than threads, FP32 activations, 8-bit codes, and biases that do not follow the scales (the bias product
+on its own). The option expert_kernels names them, so that no case runs on the item kernels unnoticed."""
 import numpy as np
 import pytest
 
@@ -20,11 +21,14 @@ TOL = 2e-3          # max-abs error over the output's RMS, the specification's b
     (40, dict(hidden=3072, experts=64)),
     (33, dict(hidden=384, ffn=128, experts=32)),                         # six groups; a row of 64 code bytes
     (70, dict(hidden=2560, ffn=640, experts=64, meta_dtype=BF16)),       # ten groups: an odd number of stages, half of the last one
-    (70, dict(hidden=1280, ffn=384, experts=64, act_dtype=F32)),         # two FP16 terms per activation, five pairs of 20 groups
+    (70, dict(hidden=1280, ffn=384, experts=64, act_dtype=F32)),         # two FP16 terms per activation, three pairs of which the last has one stage
     (130, dict(hidden=512, ffn=256, experts=32)),                        # items of about forty rows
     (5000, dict(hidden=128, ffn=128, experts=32, top_k=8, act_dtype=F32)),   # 5,600 passes: more than a table of 32 per CTA
     (45, dict(hidden=2048, experts=64, down_bits=8, q8_signed=1)),
     (45, dict(hidden=640, ffn=128, experts=32, gate_bits=8, up_bits=8, down_bits=8)),
+    (30, dict(hidden=2048, experts=64, gate_bits=8, up_bits=8, down_bits=4)),
+    (200, dict(hidden=256, ffn=128, experts=1024, top_k=8)),             # two list entries per thread
+    (40, dict(hidden=4096, experts=32, act_dtype=F32)),                  # one row block of two terms, eight warps of their own tiles
     (64, dict(hidden=2560, ffn=640, experts=64, meta_dtype=BF16, act_dtype=F32, router_dtype=BF16, arith=ARITH_REFERENCE)),
 ])
 def test_streamed_experts_against_the_checker(tokens, kw):
@@ -39,7 +43,12 @@ def test_streamed_experts_against_the_checker(tokens, kw):
     m = Moe(cfg, 0)
     w, gate = synth.router(cfg, SEED, 0), synth.shared_gate(cfg, SEED, 0)
     m.load_layer(0, np.stack(records), router_w=w, shared_record=shared, shared_gate_w=gate)
+    m.set_option("expert_kernels", 2)
     x = synth.activations(cfg, SEED, 0, tokens)
+    if cfg.gate_bits > cfg.down_bits:
+        # 8-bit gate and up weights reach 2.5: activations of 1/16 keep the SwiGLU rows inside the 4-bit down projection's range
+        x = x / 16
+        assert max(np.abs(oracle.expert(cfg.as_dict(), r, x)[0]).max() for r in records + [shared]) < 4094
     dev = torch.from_numpy(x).to(device="cuda", dtype=m.act_torch)
     got = m.decode(0, dev)
     assert m.status() == 0
@@ -52,12 +61,14 @@ def test_streamed_experts_against_the_checker(tokens, kw):
     assert torch.equal(m.decode(0, dev), got)
 
 
-def test_a_token_does_not_depend_on_its_place_in_the_batch():
+@pytest.mark.parametrize("kernels", [1, 2])
+def test_a_token_does_not_depend_on_its_place_in_the_batch(kernels):
     torch = pytest.importorskip("torch")
     from zerocool_b200.moe import Moe
     cfg = util.cfg2(experts=64, max_tokens=200)
     m = Moe(cfg, 0)
     m.synth_fill_layer(0, SEED)
+    m.set_option("expert_kernels", kernels)
     x = torch.from_numpy(synth.activations(cfg, SEED, 0, 200)).to(device="cuda", dtype=torch.bfloat16)
     order = torch.from_numpy(np.random.default_rng(3).permutation(200)).cuda()
     assert torch.equal(m.decode(0, x)[order], m.decode(0, x[order].contiguous()))
