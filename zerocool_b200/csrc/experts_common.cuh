@@ -74,31 +74,25 @@ __device__ __forceinline__ void dequant_q8(uint32_t w, bool is_signed, uint32_t 
 // than odd slots / 16, which keeps small activations out of FP16's subnormal range; the accumulated result is multiplied by 1/16
 // (exact) when it is finished. The bias term multiplies the sum of the activations. Outside the reference arithmetic it uses the
 // sum of the values the MMA really sees, so that a rounding of an activation to FP16 enters the result through the weight s q + b
-// and not through s q alone. most: the largest magnitude staged so far.
+// and not through s q alone. beyond: some value would become an FP16 infinity (reported, not hidden).
 template <bool Q4ORDER, bool SPLIT, bool FOLD>
-__device__ __forceinline__ void convert8(const float (&v)[8], bool ref, uint4& hi, uint4& lo, float& sx, float& sf, float& most) {
+__device__ __forceinline__ void convert8(const float (&v)[8], bool ref, uint4& hi, uint4& lo, float& sx, float& sf, bool& beyond) {
     sx = sf = 0.0f;
     if (ref) sx = bf_round(bf_round(bf_round(v[0] + v[1]) + v[2]) + v[3]) + bf_round(bf_round(bf_round(v[4] + v[5]) + v[6]) + v[7]);
     constexpr float EVEN = (FOLD && Q4ORDER) ? 16.0f : 1.0f;
     constexpr int order_q4[8] = {0, 4, 1, 5, 2, 6, 3, 7};
-    alignas(16) __half2 h[4], l[4];
-    float sn = 0.0f, fed[8];               // sums of the values as fed to the MMA, k ascending: as staged (sf), and in natural scale
+    __half h[8], l[8];
+    float sn = 0.0f;                       // sums of the values as fed to the MMA, k ascending: as staged (sf), and in natural scale
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int a = Q4ORDER ? order_q4[2 * i] : 2 * i, b = Q4ORDER ? order_q4[2 * i + 1] : 2 * i + 1;
-        const float va = (a & 1) ? v[a] : v[a] * EVEN, vb = (b & 1) ? v[b] : v[b] * EVEN;
-        most = fmaxf(most, fmaxf(fabsf(va), fabsf(vb)));
-        h[i] = __floats2half2_rn(va, vb);
-        float2 f = __half22float2(h[i]);
-        if (SPLIT) {
-            l[i] = __floats2half2_rn(va - f.x, vb - f.y);
-            const float2 low = __half22float2(l[i]);
-            f.x += low.x; f.y += low.y;
-        }
-        fed[a] = f.x; fed[b] = f.y;
+    for (int i = 0; i < 8; ++i) {
+        const float pre = (i & 1) ? v[i] : v[i] * EVEN;
+        beyond |= fabsf(pre) > 65504.0f;
+        h[i] = __float2half_rn(pre);
+        float fed = __half2float(h[i]);
+        if (SPLIT) { l[i] = __float2half_rn(pre - fed); fed += __half2float(l[i]); }
+        sf += fed;
+        sn += (i & 1) ? fed : fed * (1.0f / EVEN);
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { sf += fed[i]; sn += (i & 1) ? fed[i] : fed[i] * (1.0f / EVEN); }
     if (!ref) sx = sn;
 #pragma unroll
     for (int off = 1; off <= 4; off <<= 1) {
@@ -106,8 +100,15 @@ __device__ __forceinline__ void convert8(const float (&v)[8], bool ref, uint4& h
         if (FOLD) sf += __shfl_xor_sync(0xffffffffu, sf, off);
     }
     if (FOLD && Q4ORDER) sx *= 16.0f;
-    hi = *reinterpret_cast<const uint4*>(h);
-    if (SPLIT) lo = *reinterpret_cast<const uint4*>(l);
+    uint32_t ph[4], pl[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int a = Q4ORDER ? order_q4[2 * i] : 2 * i, b = Q4ORDER ? order_q4[2 * i + 1] : 2 * i + 1;
+        ph[i] = uint32_t(__half_as_ushort(h[a])) | (uint32_t(__half_as_ushort(h[b])) << 16);
+        if (SPLIT) pl[i] = uint32_t(__half_as_ushort(l[a])) | (uint32_t(__half_as_ushort(l[b])) << 16);
+    }
+    hi = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+    if (SPLIT) lo = make_uint4(pl[0], pl[1], pl[2], pl[3]);
 }
 
 }  // namespace

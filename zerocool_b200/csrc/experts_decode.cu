@@ -146,7 +146,7 @@ template <bool Q4ORDER, bool SPLIT, bool FOLD, typename RowOf>
 __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, RowOf row_of, uint32_t nvalid, uint32_t K, uint32_t RS, uint32_t GP,
                                            bool ref, __half* hi, __half* lo, float* sx_out, float* offs, uint32_t* status, uint32_t first, uint32_t stride) {
     const uint32_t per_row = (K + 255) / 256, lane = threadIdx.x % 32;
-    float most = 0.0f;
+    bool beyond = false;
     uint32_t n = 0, piece = first;
     while (n < nvalid) {
         while (piece >= per_row) { piece -= per_row; ++n; }
@@ -170,7 +170,7 @@ __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, RowOf 
         }
         uint4 ph, pl;
         float sx, sf;
-        convert8<Q4ORDER, SPLIT, FOLD>(v, ref, ph, pl, sx, sf, most);
+        convert8<Q4ORDER, SPLIT, FOLD>(v, ref, ph, pl, sx, sf, beyond);
         if (live) {
             if ((lane & 7) == 0) {
                 sx_out[n * GP + q / 8] = sx;
@@ -184,7 +184,7 @@ __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, RowOf 
         }
         piece += stride;
     }
-    if (!(most <= 65504.0f)) atomicOr(status, ZC_STATUS_RANGE);        // would become an FP16 infinity: reported, not hidden
+    if (beyond) atomicOr(status, ZC_STATUS_RANGE);
 }
 
 // d[m] (16 rows x 8 tokens) = off + sum over one 64-wide group of code * x, for the two 16-row fragments m of a stage (the
@@ -789,19 +789,19 @@ static double expected_passes(double rows, double experts) {
 // Batches that stay with the item kernels (csrc/experts_item.cu), whose many small CTAs start faster. The figures are item / streaming,
 // us a layer, for loads that fall evenly; `rounds` is how often a launch's gate/up tiles fill the streaming kernel's warps.
 //  - Up to 64 rows and tokens the item kernels split K over eight warps and win while there is little to stream: 0.36 rounds (2 tokens
-//    of 512 experts 35.9 / 37.0, hidden 2560 44.2 / 47.3; 3 tokens of 256 experts 34.3 / 34.1, hidden 2560 45.7 / 46.1), 0.17 rounds with
-//    two-term rows (2 tokens, FP32 activations: streaming 8 - 10 % faster) and above hidden 2560 (hidden 3072: 1 token 37.0 / 39.1, 2 tokens
-//    52.9 / 46.6; hidden 4096: 1 token 44.3 / 45.5 launched one by one though 44.7 / 44.1 from a graph, 2 tokens 61.9 / 52; the shared expert
+//    of 512 experts 35.5 / 37.0, hidden 2560 44.2 / 47.5; 3 tokens of 256 experts 35.2 / 35.1, hidden 2560 43.7 / 44.0), 0.17 rounds with
+//    two-term rows (2 tokens, FP32 activations: streaming 8 - 10 % faster) and above hidden 2560 (hidden 3072: 1 token 36.3 / 38.8, 2 tokens
+//    51.4 / 45.4; hidden 4096: 1 token 44.3 / 45.5 launched one by one though 44.2 / 44.0 from a graph, 2 tokens 62.5 / 52.5; the shared expert
 //    alone 12.0 / 18.5).
 //  - Beyond, where a round of the streaming kernel is nearly empty and few experts need a second pass: 1.7 to 1.97 rounds (14 / 15 / 16 /
-//    17 tokens 78.2 / 77.2, 78.2 / 78.6, 78.6 / 80.7, 91.5 / 88.9; 14 tokens at ffn 768 of 256 experts 73.3 / 78.8). With a down
+//    17 tokens 77.7 / 77.0, 78.2 / 78.6, 78.6 / 80.7, 91.5 / 88.9; 14 tokens at ffn 768 of 256 experts 73.3 / 78.8). With a down
 //    projection whose K is not whole stages (ffn 640: ten groups cost twelve) the streaming kernel loses more often: 0.8 to 2.5
 //    rounds, except from 0.47 to 0.82 of a round (512 experts of 2560 / 640: 8 tokens 76.4 / 83.0, 10 tokens 93 / 93, 14 tokens 107.7 /
-//    112.4, 18 tokens 130.2 / 128.8; 64 experts: 24 tokens 70.0 / 72.3, 48 tokens 83.6 / 80.4). Skewed loads (Zipf 1.1) would be better
+//    112.4, 18 tokens 130.2 / 128.8; 64 experts: 24 tokens 70.0 / 72.3, 48 tokens 84.0 / 80.8). Skewed loads (Zipf 1.1) would be better
 //    off streaming there: 16 tokens 72.8 / 54.8, at 2560 / 640 72.2 / 69.8. Above 2.5 rounds even loads gain 1 to 2 % on the item
 //    kernels (22 tokens 145.9 / 149.0) and skewed ones lose 10 (89.4 / 80.9): those batches stream.
 //  - Experts with more rows take further passes, and the codes are dequantised for each: there the streaming kernel
-//    wins (128 experts: 64 tokens 84 / 81, 128 tokens 124 / 114; 512 experts with skewed loads, 64 tokens 302 / 87).
+//    wins (128 experts: 64 tokens 83.8 / 80.6, 128 tokens 119.5 / 109.9; 512 experts with skewed loads, 64 tokens 302 / 87).
 bool item_kernels_pay(const ExpertLoad& l, uint32_t sms) {
     const double passes = expected_passes(l.rows, l.experts) + (l.shared_tokens + NROW - 1) / NROW;
     const double rounds = passes * (l.ffn / 16) / (double(sms) * MAX_WARPS);

@@ -1,6 +1,6 @@
 // Decode family, item kernels: the routed and shared experts with one CTA per item and row tiles, for the batches
-// that these many small CTAs finish first (one or two tokens, and a band of short batches; experts_decode.cu has the rule and
-// both sides' times) and for record geometries TMA cannot describe. The other batches stream through experts_decode.cu.
+// that these many small CTAs finish first (one or two tokens, and some short batches; experts_decode.cu has the rule and
+// both sides' times) and for handles whose records have no TMA view. The other batches stream through experts_decode.cu.
 //
 // Replaces, for every expert that received work, the reference's per-expert launches
 //   gated_linear -> q4_gate_mv_r2 / q4_gate_up (kernels/metal/qwen.metal:333-376, 71-81)
@@ -119,7 +119,7 @@ template <bool Q4ORDER, bool SPLIT, bool FOLD>
 __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, const int* rows, uint32_t nvalid,
                                            uint32_t K, bool ref, __half* hi, __half* lo, float* sums, uint32_t* status) {
     const uint32_t RS = K + ROW_PAD, blocks = K / 8, total = nvalid * blocks;
-    float most = 0.0f;
+    bool beyond = false;
     // The trip count is uniform per warp (the shuffles below need all 32 lanes); lanes past the end carry zeros.
     for (uint32_t idx = threadIdx.x; (idx & ~31u) < total; idx += EXPERT_THREADS) {
         const bool live = idx < total;
@@ -141,13 +141,13 @@ __device__ __forceinline__ void stage_rows(const void* src, bool src_f32, const 
         }
         uint4 ph, pl;
         float sx, sf;
-        convert8<Q4ORDER, SPLIT, FOLD>(v, ref, ph, pl, sx, sf, most);
+        convert8<Q4ORDER, SPLIT, FOLD>(v, ref, ph, pl, sx, sf, beyond);
         if (!live) continue;
         if ((q & 7) == 0) *reinterpret_cast<float2*>(sums + ((q / 8) * NTOK + n) * 2) = make_float2(sx, FOLD ? -1024.0f * sf : 0.0f);
         *reinterpret_cast<uint4*>(hi + n * RS + q * 8) = ph;
         if (SPLIT) *reinterpret_cast<uint4*>(lo + n * RS + q * 8) = pl;
     }
-    if (!(most <= 65504.0f)) atomicOr(status, ZC_STATUS_RANGE);        // would become an FP16 infinity: reported, not hidden
+    if (beyond) atomicOr(status, ZC_STATUS_RANGE);
 }
 
 // Source of one matrix for this lane's cp.async copies. A pass of the warp copies ROWS_PER_PASS rows: the
@@ -187,9 +187,11 @@ __device__ __forceinline__ void issue_matrix(uint32_t stage, uint32_t meta_area,
     for (int p = 0; p < F::PASSES; ++p)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(stage + src.dst0 + p * F::ROWS_PER_PASS * F::LINE),
                      "l"(g0 + size_t(p * F::ROWS_PER_PASS) * src.row_bytes) : "memory");
-    const uint32_t to = meta_area + slot * (32 * CHT * 2) + src.meta_pair * CHT * 2;
-    if constexpr (CHT == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(src.tile_meta + grp0 * 2) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(src.tile_meta + grp0 * 2) : "memory");
+    if constexpr (CHT == 4) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(meta_area + slot * (32 * CHT * 2) + src.meta_pair * CHT * 2), "l"(src.tile_meta + grp0 * 2) : "memory");
+    } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(meta_area + slot * (32 * CHT * 2) + src.meta_pair * CHT * 2), "l"(src.tile_meta + grp0 * 2) : "memory");
+    }
 }
 
 // d(16 rows x 8 tokens) = sum over one 64-wide group of code * x for the lane's rows g (w0) and g+8 (w1).
@@ -350,7 +352,8 @@ __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN
                 cp_async_wait<STAGES - 2>();
                 __syncwarp();
                 const uint8_t* stage = my_ring + slot * STAGE;
-                const uint8_t* mbase = my_meta + slot * (32 * CH * 2);                            // this chunk's scale and bias halves
+                constexpr uint32_t PAIR = uint32_t(CH * 2);                              // bytes of one (row, kind) entry
+                const uint8_t* mbase = my_meta + slot * (32 * CH * 2);                  // this chunk's scale and bias halves
                 slot = slot + 1 == STAGES ? 0 : slot + 1;
                 issue();          // refills the slot consumed by the previous iteration while this chunk is multiplied
                 const uint32_t grp0 = (ks + i * KS) * CH;
@@ -359,9 +362,9 @@ __global__ void __launch_bounds__(EXPERT_THREADS, NMAT == 1 ? ZC_MIN_BLOCKS_DOWN
                 for (int m = 0; m < WM; ++m) {
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
-                        const uint8_t* mp = mbase + m * META_AREA + (g + 8 * r) * 4 * CH;
+                        const uint8_t* mp = mbase + m * META_AREA + (g + 8 * r) * 2 * PAIR;
                         if constexpr (CH == 4) {
-                            const uint2 sc = *reinterpret_cast<const uint2*>(mp), bi = *reinterpret_cast<const uint2*>(mp + 2 * CH);
+                            const uint2 sc = *reinterpret_cast<const uint2*>(mp), bi = *reinterpret_cast<const uint2*>(mp + PAIR);
                             mraw[m][r][0] = sc.x; mraw[m][r][1] = sc.y; mraw[m][r][2] = bi.x; mraw[m][r][3] = bi.y;
                         } else {
                             const uint2 v = *reinterpret_cast<const uint2*>(mp);
