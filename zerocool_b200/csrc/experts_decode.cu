@@ -11,11 +11,11 @@
 //
 // Each launch streams every selected record once per eight rows (a pass). What bounds it is HBM as long as a weight costs few
 // enough instructions: at 6.5 TB/s an SM receives ~46 4-bit weights per clock and can issue four warp instructions, so 1,024
-// weights (16 rows x 64 k, one quantisation group of a tile) have ~88 issue slots at best. The item kernels spend 82
-// instructions on them (ncu), this one 57, 36 of which are the product itself; in mid-launch a warp's 1,024 weights take
-// 23.4 clocks of its SM, against 22 at the copy bandwidth. Layers measured against the item kernels (us): 5 tokens 58 -> 49,
-// 64 tokens 176 -> 170, 160 tokens 254 -> 231, 400 tokens 405 -> 349, 256 tokens at hidden 4096 605 -> 492; 700 tokens with
-// Zipf-skewed loads 1816 -> 438 (the passes of one long item are spread over the machine instead of two CTAs).
+// weights (16 rows x 64 k, one quantisation group of a tile) have ~88 issue slots at best. With everything around the products
+// the item kernels execute 68 instructions on them (ncu, gate/up at 64 tokens), this one 61. Layers measured against the item
+// kernels (us): 5 tokens 59 -> 50, 64 tokens 181 -> 172, 128 tokens 241 -> 231, 256 tokens 304 -> 264, 256 tokens at hidden 4096
+// 605 -> 484; 700 tokens with Zipf-skewed loads 1816 -> 438 (the passes of one long item are spread over the machine instead of two CTAs).
+// The 4-bit instantiations use all 128 registers a thread can have here and spill 4 to 48 bytes, the 8-bit ones with two-term rows 82 to 106.
 // What is left at 64 tokens: ~8 us per launch until the first product (item list, tables, rows, then the first 128 KB per SM),
 // and ends of the CTAs' runs that differ by up to a tenth.
 //  * The multiply-accumulates run on the tensor cores as m16n8k16 FP16 MMAs with up to eight token
