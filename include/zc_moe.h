@@ -225,7 +225,8 @@ int zc_moe_forward_routed(zc_moe* moe, uint32_t layer, const void* x, uint32_t t
  *     n_rows <= max_tokens * top_k * ranks.
  *   zc_moe_ep_combine: y_sorted [tokens*K, H] fp32 — the results of this rank's own rows, returned by the
  *     reverse all-to-all in the order zc_moe_ep_dispatch wrote them — is scattered to the router slots and
- *     reduced in fixed slot order with the locally computed shared expert into out. */
+ *     reduced in fixed slot order with the locally computed shared expert into out. The slots are those of the handle's last
+ *     zc_moe_ep_dispatch; one that this call's tokens do not have is left out and raises ZC_STATUS_INVALID_ROUTE. */
 int zc_moe_ep_dispatch(zc_moe* moe, uint32_t layer, const void* x, uint32_t tokens, void* rows, int32_t* row_experts, void* stream);
 int zc_moe_ep_experts(zc_moe* moe, uint32_t layer, const void* rows, const int32_t* row_experts, uint32_t n_rows, float* y, void* stream);
 int zc_moe_ep_combine(zc_moe* moe, uint32_t layer, const void* x, uint32_t tokens, const float* y_sorted, void* out, void* stream);

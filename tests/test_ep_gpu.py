@@ -102,3 +102,18 @@ def test_two_process_nccl_run():
     r = subprocess.run(cmd, capture_output=True, text=True, timeout=300, env=env, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     assert "ep ok" in r.stdout
+
+
+def test_combine_of_another_batch_than_the_dispatched_one_is_reported():
+    """ep_combine scatters by the permutation of the last ep_dispatch. Slots that the call does not have are not written (here
+    they would still lie inside the handle's buffers) and raise the invalid-route bit."""
+    import torch
+    m = make(util.cfg2(experts=64, local_experts=32, max_tokens=64))
+    m.synth_fill_layer(0, SEED)
+    x = device_x(m, synth.activations(m.cfg, SEED, 0, 9))
+    y = torch.zeros(90, m.cfg.hidden, device="cuda")
+    m.ep_dispatch(0, x)
+    m.ep_combine(0, x, y)
+    assert m.status() == 0
+    m.ep_combine(0, x[:4].contiguous(), y[:40].contiguous())
+    assert m.status() == 1

@@ -141,11 +141,13 @@ __global__ void ep_gather_kernel(const void* __restrict__ x, uint32_t row_bytes,
     if (threadIdx.x == 0) row_experts[i] = ids[slot];
 }
 
-// expert_out[perm[i], :] = y[i, :] for i < offsets[E].
+// expert_out[perm[i], :] = y[i, :] for i < offsets[E]. The permutation is the one that the last dispatch left in the handle: a slot
+// beyond this call's (another batch, or no dispatch at all) is reported and not written.
 __global__ void ep_scatter_kernel(const float* __restrict__ y, const int32_t* __restrict__ perm, const int32_t* __restrict__ offsets, uint32_t E,
-                                  uint32_t H, float* __restrict__ expert_out) {
+                                  uint32_t H, float* __restrict__ expert_out, uint32_t* __restrict__ status) {
     const uint32_t i = blockIdx.x;
     if (i >= uint32_t(offsets[E])) return;
+    if (uint32_t(perm[i]) >= gridDim.x) { if (threadIdx.x == 0) atomicOr(status, ZC_STATUS_INVALID_ROUTE); return; }
     const float4* src = reinterpret_cast<const float4*>(y + size_t(i) * H);
     float4* dst = reinterpret_cast<float4*>(expert_out + size_t(uint32_t(perm[i])) * H);
     for (uint32_t j = threadIdx.x; j < H / 4; j += blockDim.x) dst[j] = src[j];
@@ -170,7 +172,7 @@ int launch_ep_gather(zc_moe* m, const Call& c, void* rows, int32_t* row_experts,
 
 int launch_ep_scatter(zc_moe* m, const Call& c, const float* y, cudaStream_t s) {
     Timed t(m, s, KERNEL_EP);
-    ep_scatter_kernel<<<c.T * c.K, 128, 0, s>>>(y, c.perm, c.offsets, c.E, c.H, c.expert_out);
+    ep_scatter_kernel<<<c.T * c.K, 128, 0, s>>>(y, c.perm, c.offsets, c.E, c.H, c.expert_out, c.status);
     int rc = check_launch(m, "ep scatter");
     return rc < 0 ? rc : 1;
 }
